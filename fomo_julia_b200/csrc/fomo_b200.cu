@@ -348,6 +348,7 @@ Launch launch_shape(int nx, int nz, int nbc, bool iso, bool fs) {
 
 void fill_common(fomo::StepParams& P, const Medium& m, const Shot& s) {
     std::memset(&P, 0, sizeof(P));
+    P.neg_zero = -0.f;
     P.nx = m.nx;
     P.nz = m.nz;
     P.pitch = m.pitch;
@@ -1575,6 +1576,7 @@ extern "C" int fomo_b200_run_shot_noalloc(int32_t nx, int32_t nz, int32_t M, int
 
     fomo::StepParams P;
     std::memset(&P, 0, sizeof(P));
+    P.neg_zero = -0.f;
     P.nx = nx;
     P.nz = nz;
     P.pitch = pitch;

@@ -690,6 +690,7 @@ class Server {
 
         fomo::StepParams P;
         std::memset(&P, 0, sizeof(P));
+        P.neg_zero = -0.f;
         P.nx = m.nx;
         P.nz = m.nz;
         P.pitch = m.pitch;

@@ -50,6 +50,7 @@ struct StepParams {
     float* gather;              // [nt x n_rec] column major
     int tiles_x, tiles_z;       // tile grid of the cell pass
     int n_tile_blocks, n_band_blocks;
+    float neg_zero;             // -0.f, the addend of packed products (mul2)
 };
 
 __device__ __forceinline__ float fadd(float a, float b) { return __fadd_rn(a, b); }
