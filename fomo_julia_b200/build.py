@@ -20,7 +20,7 @@ CSRC = os.path.join(HERE, "csrc")
 OUT_DIR = os.path.join(HERE, "_lib")
 OBJ_DIR = os.path.join(OUT_DIR, "obj")
 LIB = os.path.join(OUT_DIR, "libfomo_b200.so")
-SOURCES = ["fomo_b200.cu", "march_m1.cu", "march_m2.cu", "march_m3.cu", "march_m4.cu"]
+SOURCES = ["fomo_b200.cu", *[f"march_m{m}.cu" for m in range(1, 5)], *[f"resident_m{m}.cu" for m in range(1, 7)]]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 FLAGS = ["-O3", "-std=c++17", "-lineinfo", "--fmad=false", "-Xcompiler", "-fPIC,-O2", "--expt-relaxed-constexpr"]
 

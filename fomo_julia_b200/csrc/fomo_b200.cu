@@ -26,6 +26,7 @@
 #include "../../include/fomo_b200.h"
 #include "step_tiled.cuh"
 #include "march_launch.h"
+#include "resident_launch.h"
 #include "step_march.cuh"
 
 namespace {
@@ -139,6 +140,9 @@ struct Context {
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     int* d_status = nullptr;   // device error word of the kernels, then the fused step's work queue (2 ints)
     cudaMemPool_t pool = nullptr;
+    ulonglong2* mail = nullptr;  // mailboxes of the resident kernel, and their number of messages
+    size_t mail_items = 0;
+    uint32_t mail_tag = 1;       // tag of the next resident step (0: never sent)
     uint64_t next = 1;
     std::unordered_map<uint64_t, std::unique_ptr<Object>> objs;
 };
@@ -402,6 +406,7 @@ int check_status() {
     CUDA_TRY(cudaMemcpyAsync(&st, ctx().d_status, sizeof(int), cudaMemcpyDeviceToHost, ctx().stream));
     CUDA_TRY(cudaStreamSynchronize(ctx().stream));
     if (st == fomo::kErrTmaTimeout) return fail(FOMO_ETIMEOUT, "a TMA load of a time-step kernel did not complete");
+    if (st == fomo::kErrResidentTimeout) return fail(FOMO_ETIMEOUT, "a block of the resident kernel did not hear from its neighbours");
     if (st) return fail(FOMO_ECUDA, "time-step kernel reported error %d", st);
     return FOMO_OK;
 }
@@ -596,6 +601,88 @@ int run_steps_march(Shot& s, Medium& m, Wavefield& w, int n_steps, Profile* prof
     return check_status();
 }
 
+// ---------------------------------------------------------------- resident steps
+// Blocks of the resident kernel the device holds at once (0: none).
+template <int M>
+int resident_slots(size_t smem, int h_max) {
+    const void* fn = fomo::resident_kernel_fn<M>(h_max);
+    int per_sm = 0;
+    if (raise_smem_limit(fn, smem) != FOMO_OK ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, fomo::kRThreads, smem) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return 0;
+    }
+    return per_sm * sm_count();
+}
+
+// The resident kernel's plan of a shot's grid.
+template <int M>
+fomo::ResidentPlan shot_resident_plan(const Shot& s, const Medium& m) {
+    fomo::ResidentPlan p = fomo::resident_plan(m.nx, m.nz, M, s.nbc, m.fs != 0, s.dtx == s.dtz, sm_count());
+    if (p.ok && resident_slots<M>(p.smem, p.L.h_max) < p.L.strips * p.L.rows) p.ok = false;
+    return p;
+}
+
+template <int M>
+int run_steps_resident(Shot& s, Medium& m, Wavefield& w, int n_steps, const fomo::ResidentPlan& plan) {
+    auto& C = ctx();
+    if (int rc = ensure_buoyancy(m, s.dtx, s.dtz)) return rc;
+    const int blocks = plan.L.strips * plan.L.rows;
+    const size_t items = (size_t)blocks * fomo::resident_mail_items(M, plan.L.h_max);
+    // Messages carry the step's tag, which only grows: a mailbox is cleared
+    // when it is allocated and when the tags wrap.
+    if (items > C.mail_items) {
+        pool_free(C.mail);
+        C.mail = nullptr;
+        C.mail_items = 0;
+        const cudaError_t e = pool_alloc((void**)&C.mail, items * sizeof(ulonglong2));
+        if (e != cudaSuccess) return fail(FOMO_ENOMEM, "mailbox allocation failed: %s", cudaGetErrorString(e));
+        C.mail_items = items;
+        CUDA_TRY(cudaMemsetAsync(C.mail, 0, items * sizeof(ulonglong2), C.stream));
+    }
+    fomo::ResidentArgs A;
+    std::memset(&A, 0, sizeof(A));
+    A.L = plan.L;
+    buoyancy_ptrs(m, A.b);
+    A.iso = s.dtx == s.dtz ? 1 : 0;
+    A.status = C.d_status;
+    A.mail = C.mail;
+    CUDA_TRY(cudaEventRecord(C.ev0, C.stream));
+    const int k_end = std::min(s.nt, s.k_done + n_steps);
+    nvtxRangePushA("fomo_b200 time loop (resident)");
+    for (int k = s.k_done + 1; k <= k_end;) {
+        const int n = std::min(fomo::kRMaxSteps, k_end - k + 1);
+        if (C.mail_tag > UINT32_MAX - 2 * fomo::kRMaxSteps) {
+            CUDA_TRY(cudaMemsetAsync(C.mail, 0, C.mail_items * sizeof(ulonglong2), C.stream));
+            C.mail_tag = 1;
+        }
+        const int a = w.cur, b = 1 - w.cur;
+        fomo::StepParams P;
+        fill_common(P, m, s);
+        for (int q = 0; q < 5; ++q) {
+            P.in[q] = w.field(a, q);
+            P.out[q] = w.field(b, q);
+        }
+        A.tag0 = C.mail_tag;
+        A.n_steps = n;
+        A.k0 = k;
+        for (int q = 0; q < n; ++q) A.wav[q] = k + q <= (int)s.wavelet.size() ? s.wavelet[k + q - 1] : 0.f;
+        C.mail_tag += n;
+        CUDA_TRY(fomo::resident_launch<M>(blocks, plan.smem, C.stream, P, A));
+        s.launches += 1;
+        w.cur = b;
+        k += n;
+        s.k_done = s.recorded = k - 1;
+    }
+    nvtxRangePop();
+    CUDA_TRY(cudaEventRecord(C.ev1, C.stream));
+    CUDA_TRY(cudaEventSynchronize(C.ev1));
+    float ms = 0;
+    CUDA_TRY(cudaEventElapsedTime(&ms, C.ev0, C.ev1));
+    s.device_ms += ms;
+    return check_status();
+}
+
 // The fused step's plan for a shot, or !ok (split launches): FOMO_STEP_SPLIT,
 // M > 4, or a layout march_plan rejects.
 template <int M>
@@ -665,9 +752,25 @@ void save_step_choice(const StepKey& k, int c) {
     }
 }
 
+// Records, once per process and grid, that a grid does not run the fused step
+// (it runs the resident kernel, which needs no timing).
+void note_step_choice(const StepKey& k) {
+    if (k.M > 4 || !k.fs) return;  // the fused step never applies there: nothing to choose
+    std::lock_guard<std::mutex> lk(g_step_choice_mu);
+    load_step_choices();
+    if (g_step_choice.emplace(k, 0).second) save_step_choice(k, 0);
+}
+
 template <int M>
 int run_steps_M(Shot& s, Medium& m, Wavefield& w, int n_steps, Profile* prof) {
     const int mode = g_step_mode.load();
+    if (mode == FOMO_STEP_AUTO && !prof) {
+        const fomo::ResidentPlan res = shot_resident_plan<M>(s, m);
+        if (res.ok) {
+            note_step_choice(StepKey{m.nx, m.nz, M, s.nbc, m.fs, s.dtx == s.dtz});
+            return run_steps_resident<M>(s, m, w, n_steps, res);
+        }
+    }
     const MarchPlan plan = shot_march_plan<M>(s, m);
     if (!plan.ok) {
         if (mode == FOMO_STEP_FUSED) return fail(FOMO_EINVAL, "the fused step does not support this shot: %s", plan.why);
@@ -878,6 +981,9 @@ int fomo_b200_shutdown(void) {
     if (!C.inited) return FOMO_OK;
     cudaStreamSynchronize(C.stream);
     C.objs.clear();
+    pool_free(C.mail);
+    C.mail = nullptr;
+    C.mail_items = 0;
     cudaStreamSynchronize(C.stream);
     cudaMemPoolDestroy(C.pool);
     C.pool = nullptr;

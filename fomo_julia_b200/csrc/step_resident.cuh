@@ -1,0 +1,793 @@
+// step_resident.cuh -- many time steps of one shot in one launch, for grids
+// whose five fields fit the chip's shared memory.
+//
+// What bounds small grids is latency, not bytes: a step of the split launches
+// is four dependent launches, each of them one or two waves of tiles that
+// load, compute and store once.  Here each block owns a region of the grid
+// (up to 64 columns, any number of rows) and keeps its five fields, with an
+// M-cell halo, in shared memory for all the steps of the launch.  A half step
+// reads and writes shared memory only; the blocks then exchange the M border
+// columns and rows of the fields the next half step differentiates through
+// mailboxes in global memory (L2), and nothing else crosses the chip.  The
+// launch is cooperative, since neighbouring blocks wait for each other.
+//
+// Exchange.  A message is 16 bytes: two values, each in one 64-bit word with
+// the step's tag.  The receiver polls the words themselves until they carry
+// the tag it waits for, so an exchange costs one store and one load latency
+// and needs no fence or flag.  One mailbox per kind (v after the velocity
+// half step, tau after the stress half step) is enough: a block writes its
+// next message of a kind only after it has received its neighbours' messages
+// of the other kind, which they send after reading the previous one.  Waits
+// are bounded: a block that gives up sets the status word and leaves, and so
+// do its neighbours.
+//
+// Regions.  The first and last strip hold the side HABC bands and the columns
+// their rules read, the bottom row of blocks holds the whole bottom band and
+// the row above it, and without a free surface the top row of blocks holds
+// the whole top band and the row below, so no boundary rule crosses a block.
+//   sides   a thread's neighbours in x are in the same half warp, so the side
+//           rules run on registers and shuffles;
+//   bottom  the recurrence along j (boundary.jl:88-132) runs in the plane,
+//           one warp per field, with the step-start values in a scratch;
+//   top     pointwise on values before the band rule, kept in a scratch.
+// The source is added in the plane right after a step's stresses are final
+// (before they are sent), the values before it are kept beside for the HABC
+// and the receivers (source_receiver.jl:18-30, boundary.jl:20-56).
+#pragma once
+
+#include "resident_launch.h"
+#include "step_tiled.cuh"
+
+namespace fomo {
+
+// One 16-byte message; each half is written and read as one 64-bit access.
+__device__ __forceinline__ void mail_put(ulonglong2* p, float a, float b, uint32_t tag) {
+    const uint64_t lo = ((uint64_t)tag << 32) | __float_as_uint(a), hi = ((uint64_t)tag << 32) | __float_as_uint(b);
+    asm volatile("st.relaxed.gpu.global.v2.b64 [%0], {%1, %2};" ::"l"(p), "l"(lo), "l"(hi) : "memory");
+}
+__device__ __forceinline__ ulonglong2 mail_get(const ulonglong2* p) {
+    ulonglong2 v;
+    asm volatile("ld.relaxed.gpu.global.v2.b64 {%0, %1}, [%2];" : "=l"(v.x), "=l"(v.y) : "l"(p) : "memory");
+    return v;
+}
+constexpr int kMailPolls = 1 << 22;
+
+// z-derivatives of RT consecutive rows from a (2M + RT - 1)-row window:
+// d[rr] = sum_l a_l (w[rr+M+l-1] - w[rr+M-l]), column pairs.
+template <int M, int RT>
+__device__ __forceinline__ void zpairs(const StepParams& P, const float4 (&w)[2 * M + RT - 1], float2 (&lo)[RT],
+                                       float2 (&hi)[RT]) {
+#pragma unroll
+    for (int rr = 0; rr < RT; ++rr) {
+        float2 a = make_float2(0.f, 0.f), b = a;
+#pragma unroll
+        for (int l = 1; l <= M; ++l) {
+            const float2 al = make_float2(P.a[l - 1], P.a[l - 1]);
+            a = add2(mul2(P, al, sub2(lo2(w[rr + M + l - 1]), lo2(w[rr + M - l]))), a);
+            b = add2(mul2(P, al, sub2(hi2(w[rr + M + l - 1]), hi2(w[rr + M - l]))), b);
+        }
+        lo[rr] = a;
+        hi[rr] = b;
+    }
+}
+
+// Rows j .. j+n-1 hold a row of the side bands (a warp's rows: uniform).
+__device__ __forceinline__ bool side_rows(const StepParams& P, int j, int n) {
+    return j + n > (P.fs ? P.nbc : 1) && j <= P.nz - P.nbc - 2;
+}
+
+// What a block knows of its region.
+struct Region {
+    int x0, x1, z0, z1, h;
+    bool left, right, bottom, top, rim;
+    int si, sj;        // source, in region coordinates; sj < 0: not here
+    float* plane;      // five planes of `psize` floats, row pitch PITCH, cell (x0, z0) at M rows + HX columns
+    size_t psize;
+    float* old;        // bottom band: step-start values [3][b+1][kRW], row 0 the row above the band
+    float *e, *fin;    // top band: [3][b+3][kRW] (row b+2: step-start values of row b+1), [3][b][kRW]
+    float* tab;        // weights of vx, vz, tau by distance, b + 2 each
+    float* src;        // txx, tzz of the source cell before the source was added
+};
+
+// Side HABC of four columns x..x+3 of row j (boundary.jl:76-85) of a block on
+// one or both sides: n holds the values after the stencil update and receives
+// the final ones, o the step-start values, w the columns' weights.  All lanes
+// of the half warp that share the row call it.  edge_sum and blend_edge on
+// column pairs.
+__device__ __forceinline__ void side_rules(const StepParams& P, const Region& R, const float4& w, int x, int j, float4& n,
+                                           const float4& o) {
+    constexpr unsigned FULL = 0xffffffffu;
+    const int b = P.nbc, r0 = P.nx - b - 1;
+    const bool row = j >= (P.fs ? b : 1) && j <= P.nz - b - 2;
+    const float4 pre = n;
+    const float2 nq = make_float2(-P.qx, -P.qx), qt = make_float2(P.qt_x, P.qt_x), qxt = make_float2(P.qxt, P.qxt);
+    const float2 one = make_float2(1.f, 1.f);
+    const float2 Al = mul2(P, lo2(w), lo2(pre)), Ah = mul2(P, hi2(w), hi2(pre));
+    const float2 Wl = sub2(one, lo2(w)), Wh = sub2(one, hi2(w));
+    const float2 tl = mul2(P, qt, lo2(o)), th = mul2(P, qt, hi2(o));
+    if (R.left) {
+        const float nr = __shfl_down_sync(FULL, pre.x, 1, 16), orr = __shfl_down_sync(FULL, o.x, 1, 16);
+        const float2 sl = sub2(sub2(mul2(P, nq, make_float2(pre.y, pre.z)), tl), mul2(P, qxt, make_float2(o.y, o.z)));
+        const float2 sh = sub2(sub2(mul2(P, nq, make_float2(pre.w, nr)), th), mul2(P, qxt, make_float2(o.w, orr)));
+        const float2 fl = add2(Al, mul2(P, Wl, sl)), fh = add2(Ah, mul2(P, Wh, sh));
+        if (row && x >= 1 && x <= b) n.x = fl.x;
+        if (row && x + 1 <= b) n.y = fl.y;
+        if (row && x + 2 <= b) n.z = fh.x;
+        if (row && x + 3 <= b) n.w = fh.y;
+    }
+    if (R.right) {
+        const float nl = __shfl_up_sync(FULL, pre.w, 1, 16), ol = __shfl_up_sync(FULL, o.w, 1, 16);
+        const float2 ql = mul2(P, qxt, make_float2(ol, o.x)), qh = mul2(P, qxt, make_float2(o.y, o.z));
+        const float2 sl = sub2(sub2(mul2(P, nq, make_float2(nl, pre.x)), tl), ql);
+        const float2 sh = sub2(sub2(mul2(P, nq, make_float2(pre.y, pre.z)), th), qh);
+        float2 fl = add2(Al, mul2(P, Wl, sl)), fh = add2(Ah, mul2(P, Wh, sh));
+        // a chunk start (but the first) reads the value just computed for the column before it; the four
+        // columns hold one at most, at the same place in every lane
+        const int cs = (r0 - R.x0) & 3;
+        const float pm = __shfl_up_sync(FULL, fh.y, 1, 16);
+        const float fn = cs == 0 ? pm : cs == 1 ? fl.x : cs == 2 ? fl.y : fh.x;
+        const float t = cs == 0 ? tl.x : cs == 1 ? tl.y : cs == 2 ? th.x : th.y;
+        const float q = cs == 0 ? ql.x : cs == 1 ? ql.y : cs == 2 ? qh.x : qh.y;
+        const float A = cs == 0 ? Al.x : cs == 1 ? Al.y : cs == 2 ? Ah.x : Ah.y;
+        const float W = cs == 0 ? Wl.x : cs == 1 ? Wl.y : cs == 2 ? Wh.x : Wh.y;
+        const float f = fadd(A, fmul(W, fsub(fsub(fmul(-P.qx, fn), t), q)));
+        const int i = x + cs;
+        const bool start = i > r0 && ((i - r0) & 7) == 0;
+        if (start && cs == 0) fl.x = f;
+        if (start && cs == 1) fl.y = f;
+        if (start && cs == 2) fh.x = f;
+        if (start && cs == 3) fh.y = f;
+        if (row && x >= r0 && x <= P.nx - 2) n.x = fl.x;
+        if (row && x + 1 >= r0 && x + 1 <= P.nx - 2) n.y = fl.y;
+        if (row && x + 2 >= r0 && x + 2 <= P.nx - 2) n.z = fh.x;
+        if (row && x + 3 >= r0 && x + 3 <= P.nx - 2) n.w = fh.y;
+    }
+}
+
+// Weights of columns x..x+3 of row j from a table by distance.  Below the
+// top band they depend on the column only (every caller's row is above the
+// bottom band).
+__device__ __forceinline__ float4 side_weights(const StepParams& P, const float* tab, int x, int j) {
+    const int dj = min(j, P.nbc + 1);
+    float w[4];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) w[c] = tab[max(min(min(x + c, P.nx - 1 - x - c), dj), 0)];
+    return make_float4(w[0], w[1], w[2], w[3]);
+}
+
+template <int M>
+__device__ __forceinline__ float* cell_at(const Region& R, int q, int col, int row) {
+    return R.plane + q * R.psize + (size_t)(row + M) * resident_pitch(M) + col + resident_hx(M);
+}
+
+// Where a row's values go after the side rules.
+__device__ __forceinline__ bool in_top_rows(const StepParams& P, int j) { return !P.fs && j >= 1 && j <= P.nbc; }
+
+// Stores four columns of field f (of the half step; plane q) of row j: to the
+// plane, with the step-start values of the rows the bottom recurrence reads
+// beside; rows of the top band to its scratch, their plane keeps the
+// step-start values.
+template <int M>
+__device__ __forceinline__ void put_row(const StepParams& P, const Region& R, int f, int q, int col, int row, const float4& n,
+                                        const float4& o, bool zero, bool src_row) {
+    const int b = P.nbc, j = R.z0 + row, jb = j - (P.nz - b - 1);
+    float* p = cell_at<M>(R, q, col, row);
+    if (in_top_rows(P, j)) {
+        *reinterpret_cast<float4*>(R.e + (f * (b + 3) + j) * kRW + col) = n;
+        if (src_row) *reinterpret_cast<float4*>(p) = o;  // the band rule reads step-start values here
+        return;
+    }
+    if (jb >= -1 && jb < b) *reinterpret_cast<float4*>(R.old + (f * (b + 1) + jb + 1) * kRW + col) = o;
+    if (R.top && j == b + 1) {
+        *reinterpret_cast<float4*>(R.e + (f * (b + 3) + b + 1) * kRW + col) = n;
+        *reinterpret_cast<float4*>(R.e + (f * (b + 3) + b + 2) * kRW + col) = o;
+    }
+    *reinterpret_cast<float4*>(p) = zero ? make_float4(0.f, 0.f, 0.f, 0.f) : n;
+}
+
+// Medium of the region: global memory or its copy in shared memory.
+struct MedView {
+    const float *b0, *b1, *b2, *b3, *lam, *mu, *mxz;  // at the region's first cell
+    int pitch;
+};
+
+__device__ __forceinline__ float4 ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+
+// Stencil update and side rules of the region's velocities.
+template <int M, int RT>
+__device__ __forceinline__ void resident_velocity(const StepParams& P, const Region& R, const MedView& D) {
+    constexpr int PITCH = resident_pitch(M), HX = resident_hx(M), ROWS = kRThreads / 16 * RT;
+    const int col = 4 * (threadIdx.x & 15), x = R.x0 + col;
+#pragma unroll 1
+    for (int base = 0; base < R.h; base += ROWS) {
+        const int row = base + (threadIdx.x >> 4) * RT;
+        const bool on = row < R.h && x < R.x1;
+        float4 ox[RT], oz[RT], nx[RT], nz[RT];
+        if (on) {
+            const int mo = row * D.pitch + col;
+            float4 b0[RT], b1[RT], b2[RT], b3[RT];
+#pragma unroll
+            for (int rr = 0; rr < RT; ++rr) {
+                const int m = mo + (row + rr < R.h ? rr : 0) * D.pitch;
+                b0[rr] = ld4(D.b0 + m);
+                b2[rr] = ld4(D.b2 + m);
+                b1[rr] = D.b1 == D.b0 ? b0[rr] : ld4(D.b1 + m);
+                b3[rr] = D.b3 == D.b2 ? b2[rr] : ld4(D.b3 + m);
+            }
+            const float* xx = cell_at<M>(R, TXX, col, row) - HX;  // windows start HX columns to the left
+            const float* zz = cell_at<M>(R, TZZ, col, row);
+            const float* xz = cell_at<M>(R, TXZ, col, row);
+            float d1[RT][4], d3[RT][4];
+            float2 d2lo[RT], d2hi[RT], d4lo[RT], d4hi[RT];
+#pragma unroll
+            for (int rr = 0; rr < RT; ++rr) {
+                float w[4 * Geo<M>::NQ];
+                load_xwin<M>(xx + rr * PITCH, w);
+                xderiv<M, 0>(P, w, d1[rr]);  // dtxx/dx
+                load_xwin<M>(xz - HX + rr * PITCH, w);
+                xderiv<M, 1>(P, w, d3[rr]);  // dtxz/dx
+            }
+            {
+                float4 w[2 * M + RT - 1];
+#pragma unroll
+                for (int k = 0; k < 2 * M + RT - 1; ++k) w[k] = lds4(xz + (k - M) * PITCH);
+                zpairs<M, RT>(P, w, d2lo, d2hi);  // dtxz/dz
+#pragma unroll
+                for (int k = 0; k < 2 * M + RT - 1; ++k) w[k] = lds4(zz + (k - M + 1) * PITCH);
+                zpairs<M, RT>(P, w, d4lo, d4hi);  // dtzz/dz
+            }
+#pragma unroll
+            for (int rr = 0; rr < RT; ++rr) {
+                const float4 vx = lds4(cell_at<M>(R, VX, col, row + rr)), vz = lds4(cell_at<M>(R, VZ, col, row + rr));
+                const float2 xl = add2(lo2(vx), add2(mul2(P, lo2(b0[rr]), make_float2(d1[rr][0], d1[rr][1])), mul2(P, lo2(b1[rr]), d2lo[rr])));
+                const float2 xh = add2(hi2(vx), add2(mul2(P, hi2(b0[rr]), make_float2(d1[rr][2], d1[rr][3])), mul2(P, hi2(b1[rr]), d2hi[rr])));
+                const float2 zl = add2(lo2(vz), add2(mul2(P, lo2(b2[rr]), make_float2(d3[rr][0], d3[rr][1])), mul2(P, lo2(b3[rr]), d4lo[rr])));
+                const float2 zh = add2(hi2(vz), add2(mul2(P, hi2(b2[rr]), make_float2(d3[rr][2], d3[rr][3])), mul2(P, hi2(b3[rr]), d4hi[rr])));
+                nx[rr] = make_float4(xl.x, xl.y, xh.x, xh.y);
+                nz[rr] = make_float4(zl.x, zl.y, zh.x, zh.y);
+                ox[rr] = vx;
+                oz[rr] = vz;
+                if (R.rim) {
+#pragma unroll
+                    for (int c = 0; c < 4; ++c)
+                        if (!in_stencil(P, x + c, R.z0 + row + rr)) {
+                            set_comp(nx[rr], c, comp(vx, c));
+                            set_comp(nz[rr], c, comp(vz, c));
+                        }
+                }
+            }
+        } else {
+#pragma unroll
+            for (int rr = 0; rr < RT; ++rr) ox[rr] = oz[rr] = nx[rr] = nz[rr] = make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        if ((R.left || R.right) && side_rows(P, R.z0 + base + (threadIdx.x >> 5) * 2 * RT, 2 * RT)) {
+            __syncwarp();
+#pragma unroll
+            for (int rr = 0; rr < RT; ++rr) {
+                const int j = R.z0 + row + rr;
+                side_rules(P, R, side_weights(P, R.tab, x, j), x, j, nx[rr], ox[rr]);
+                side_rules(P, R, side_weights(P, R.tab + P.nbc + 2, x, j), x, j, nz[rr], oz[rr]);
+            }
+        }
+        if (on) {
+#pragma unroll
+            for (int rr = 0; rr < RT; ++rr)
+                if (row + rr < R.h) {
+                    put_row<M>(P, R, 0, VX, col, row + rr, nx[rr], ox[rr], false, false);
+                    put_row<M>(P, R, 1, VZ, col, row + rr, nz[rr], oz[rr], false, false);
+                }
+        }
+    }
+}
+
+// Stencil update and side rules of the region's stresses.  The planes hold
+// the source already; step-start values are those before it.
+template <int M, int RT>
+__device__ __forceinline__ void resident_stress(const StepParams& P, const Region& R, const MedView& D) {
+    constexpr int PITCH = resident_pitch(M), HX = resident_hx(M), ROWS = kRThreads / 16 * RT;
+    const int col = 4 * (threadIdx.x & 15), x = R.x0 + col;
+    const float2 dtx2 = make_float2(P.dtx, P.dtx), dtz2 = make_float2(P.dtz, P.dtz), two = make_float2(2.f, 2.f);
+#pragma unroll 1
+    for (int base = 0; base < R.h; base += ROWS) {
+        const int row = base + (threadIdx.x >> 4) * RT;
+        const bool on = row < R.h && x < R.x1;
+        float4 o0[RT], o1[RT], o2[RT], n0[RT], n1[RT], n2[RT];
+        if (on) {
+            const int mo = row * D.pitch + col;
+            float4 lam[RT], mu[RT], mxz[RT];
+#pragma unroll
+            for (int rr = 0; rr < RT; ++rr) {
+                const int m = mo + (row + rr < R.h ? rr : 0) * D.pitch;
+                lam[rr] = ld4(D.lam + m);
+                mu[rr] = ld4(D.mu + m);
+                mxz[rr] = ld4(D.mxz + m);
+            }
+            const float* vx = cell_at<M>(R, VX, col, row);
+            const float* vz = cell_at<M>(R, VZ, col, row);
+            float dxx[RT][4], dzx[RT][4];
+            float2 dzzlo[RT], dzzhi[RT], dxzlo[RT], dxzhi[RT];
+#pragma unroll
+            for (int rr = 0; rr < RT; ++rr) {
+                float w[4 * Geo<M>::NQ];
+                load_xwin<M>(vx - HX + rr * PITCH, w);
+                xderiv<M, 1>(P, w, dxx[rr]);  // dvx/dx
+                load_xwin<M>(vz - HX + rr * PITCH, w);
+                xderiv<M, 0>(P, w, dzx[rr]);  // dvz/dx
+            }
+            {
+                float4 w[2 * M + RT - 1];
+#pragma unroll
+                for (int k = 0; k < 2 * M + RT - 1; ++k) w[k] = lds4(vz + (k - M) * PITCH);
+                zpairs<M, RT>(P, w, dzzlo, dzzhi);  // dvz/dz
+#pragma unroll
+                for (int k = 0; k < 2 * M + RT - 1; ++k) w[k] = lds4(vx + (k - M + 1) * PITCH);
+                zpairs<M, RT>(P, w, dxzlo, dxzhi);  // dvx/dz
+            }
+#pragma unroll
+            for (int rr = 0; rr < RT; ++rr) {
+                const float4 txx = lds4(cell_at<M>(R, TXX, col, row + rr)), tzz = lds4(cell_at<M>(R, TZZ, col, row + rr));
+                const float4 txz = lds4(cell_at<M>(R, TXZ, col, row + rr));
+                float2 r0[2], r1[2], r2[2];
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const float2 lv = h ? hi2(lam[rr]) : lo2(lam[rr]), mv = h ? hi2(mu[rr]) : lo2(mu[rr]);
+                    const float2 l2m = add2(lv, mul2(P, two, mv));
+                    const float2 ex = mul2(P, make_float2(dxx[rr][2 * h], dxx[rr][2 * h + 1]), dtx2);
+                    const float2 ez = mul2(P, h ? dzzhi[rr] : dzzlo[rr], dtz2);
+                    r0[h] = add2(h ? hi2(txx) : lo2(txx), add2(mul2(P, l2m, ex), mul2(P, lv, ez)));
+                    r1[h] = add2(h ? hi2(tzz) : lo2(tzz), add2(mul2(P, lv, ex), mul2(P, l2m, ez)));
+                    const float2 sh = add2(mul2(P, h ? dxzhi[rr] : dxzlo[rr], dtz2),
+                                           mul2(P, make_float2(dzx[rr][2 * h], dzx[rr][2 * h + 1]), dtx2));
+                    r2[h] = add2(h ? hi2(txz) : lo2(txz), mul2(P, h ? hi2(mxz[rr]) : lo2(mxz[rr]), sh));
+                }
+                n0[rr] = make_float4(r0[0].x, r0[0].y, r0[1].x, r0[1].y);
+                n1[rr] = make_float4(r1[0].x, r1[0].y, r1[1].x, r1[1].y);
+                n2[rr] = make_float4(r2[0].x, r2[0].y, r2[1].x, r2[1].y);
+                o0[rr] = txx;
+                o1[rr] = tzz;
+                o2[rr] = txz;
+                if (R.rim) {
+#pragma unroll
+                    for (int c = 0; c < 4; ++c)
+                        if (!in_stencil(P, x + c, R.z0 + row + rr)) {
+                            set_comp(n0[rr], c, comp(txx, c));
+                            set_comp(n1[rr], c, comp(tzz, c));
+                            set_comp(n2[rr], c, comp(txz, c));
+                        }
+                }
+                if (row + rr == R.sj && R.si >= col && R.si < col + 4) {
+                    set_comp(o0[rr], R.si - col, R.src[0]);
+                    set_comp(o1[rr], R.si - col, R.src[1]);
+                }
+            }
+        } else {
+#pragma unroll
+            for (int rr = 0; rr < RT; ++rr) {
+                o0[rr] = o1[rr] = o2[rr] = make_float4(0.f, 0.f, 0.f, 0.f);
+                n0[rr] = n1[rr] = n2[rr] = o0[rr];
+            }
+        }
+        if ((R.left || R.right) && side_rows(P, R.z0 + base + (threadIdx.x >> 5) * 2 * RT, 2 * RT)) {
+            __syncwarp();
+            const float* tab = R.tab + 2 * (P.nbc + 2);
+#pragma unroll
+            for (int rr = 0; rr < RT; ++rr) {
+                const int j = R.z0 + row + rr;
+                const float4 w = side_weights(P, tab, x, j);
+                side_rules(P, R, w, x, j, n0[rr], o0[rr]);
+                side_rules(P, R, w, x, j, n1[rr], o1[rr]);
+                side_rules(P, R, w, x, j, n2[rr], o2[rr]);
+            }
+        }
+        if (on) {
+#pragma unroll
+            for (int rr = 0; rr < RT; ++rr)
+                if (row + rr < R.h) {
+                    const bool zero = in_free_surface_rows(P, R.z0 + row + rr);
+                    const bool src = row + rr == R.sj && R.si >= col && R.si < col + 4;
+                    put_row<M>(P, R, 0, TXX, col, row + rr, n0[rr], o0[rr], false, src);
+                    put_row<M>(P, R, 1, TZZ, col, row + rr, n1[rr], o1[rr], zero, src);
+                    put_row<M>(P, R, 2, TXZ, col, row + rr, n2[rr], o2[rr], zero, false);
+                }
+        }
+    }
+}
+
+// One warp's part of the bottom band's recurrence along j (rows nz-nbc-1 ..
+// nz-2) of one field, a column per lane.  `p` is the lane's column of the plane
+// at the first band row: values after the stencil update, replaced by the
+// final ones; `old` the column's step-start values, row 0 being the row above
+// the band.  A column's chain needs its own column only: five dependent
+// operations a row; loads and everything off the chain run G rows ahead.
+constexpr int kBandGroup = 5;
+template <int PITCH>
+__device__ __forceinline__ void bottom_edge(const StepParams& P, const float* tab, float* p, const float* old, bool store) {
+    constexpr int G = kBandGroup;
+    const int b = P.nbc;
+    float fp = p[-PITCH], op = old[0];
+    auto rows = [&](int g, int n) {
+        float A[G], W[G], t1[G], t2[G];
+        float* pg = p + g * PITCH;
+        const float *og = old + (g + 1) * kRW, *wg = tab + b - g;  // distance nz - 1 - j = b - jb
+#pragma unroll
+        for (int r = 0; r < G; ++r)
+            if (r < n) {
+                const float w = wg[-r], ov = og[r * kRW];
+                A[r] = fmul(w, pg[r * PITCH]);
+                W[r] = fsub(1.f, w);
+                t1[r] = fmul(P.qt_z, ov);
+                t2[r] = fmul(P.qxt, op);
+                op = ov;
+            }
+#pragma unroll
+        for (int r = 0; r < G; ++r)
+            if (r < n) {
+                fp = fadd(A[r], fmul(W[r], fsub(fsub(fmul(-P.qz, fp), t1[r]), t2[r])));
+                if (store) pg[r * PITCH] = fp;
+            }
+    };
+    int g = 0;
+#pragma unroll 1
+    for (; g + G <= b; g += G) rows(g, G);
+#pragma unroll 1
+    for (; g < b; ++g) rows(g, 1);
+}
+
+// The same near a corner, where f = A + W (sx + sz): W = (1 - w) / 2 and sx the
+// x term in a corner column, W = 1 - w and sx = -0 (which adds nothing) in an
+// edge column.  Three warps (`part`) share a field: two march the columns that
+// read their neighbour's value before the HABC, the third, one group of rows
+// behind, the columns that read its final value (the last bottom-left column
+// and the bottom-right chunk starts).  They meet at named barrier `bar` once a
+// group: every value of its rows is read before any is replaced.
+template <int PITCH>
+__device__ __forceinline__ void bottom_corner(const StepParams& P, const Region& R, const float* tab, float* p0,
+                                              const float* old0, int part, int bar) {
+    constexpr int G = kBandGroup;
+    const int lane = threadIdx.x & 31, b = P.nbc, nx = P.nx, r0 = nx - b - 1;
+    const int nr = R.right ? (b + 7) / 8 : 0;
+    const bool second = part == 2;
+    int i = second ? (lane < nr ? r0 + 8 * lane : b) : R.x0 + 32 * part + lane;
+    bool store = second ? lane < nr + (R.left ? 1 : 0) : i < min(R.x1, nx);
+    if (!store) i = R.x0;
+    const bool rim = i <= 0 || i >= nx - 1;
+    const bool lc = i >= 1 && i <= b, rc = i >= r0 && i <= nx - 2, corner = lc || rc;
+    const bool redo = (lc && i == b) || (rc && right_chunk_start(nx, b, i));
+    if (!second && redo) store = false;
+    const int dx = max(min(min(i, nx - 1 - i), b + 1), 0), dn = lc ? 1 : (rc ? -1 : 0);
+    const float h = corner ? 0.5f : 1.f;
+    float* p = p0 + (i - R.x0);
+    const float* old = old0 + (i - R.x0);
+    float fp = p[-PITCH], op = old[0];
+    auto sync = [&] { asm volatile("bar.sync %0, 96;" ::"r"(bar) : "memory"); };
+    auto rows = [&](int g, int n) {
+        float A[G], W[G], t1[G], t2[G], sx[G];
+        float* pg = p + g * PITCH;
+        const float* og = old + (g + 1) * kRW;
+#pragma unroll
+        for (int r = 0; r < G; ++r)
+            if (r < n) {
+                const float w = tab[min(dx, b - g - r)], ov = og[r * kRW], pv = pg[r * PITCH];
+                const float s = edge_sum(P.qx, P.qt_x, P.qxt, pg[r * PITCH + dn], ov, og[r * kRW + dn]);
+                sx[r] = corner ? s : -0.f;
+                A[r] = rim ? pv : fmul(w, pv);
+                W[r] = fmul(fsub(1.f, w), h);
+                t1[r] = fmul(P.qt_z, ov);
+                t2[r] = fmul(P.qxt, op);
+                op = ov;
+            }
+        if (!second) sync();
+#pragma unroll
+        for (int r = 0; r < G; ++r)
+            if (r < n) {
+                const float f = fadd(A[r], fmul(W[r], fadd(sx[r], fsub(fsub(fmul(-P.qz, fp), t1[r]), t2[r]))));
+                fp = rim ? A[r] : f;  // the grid's rim keeps its value
+                if (store) pg[r * PITCH] = fp;
+            }
+    };
+    if (second) sync();  // the first group has been read
+    int g = 0;
+#pragma unroll 1
+    for (; g < b; g += G) {
+        if (second) sync();  // the group is final but for this warp's columns
+        rows(g, min(G, b - g));
+    }
+    if (!second) sync();
+}
+
+// Bottom band of the block's columns for n_fields fields from plane q0.
+template <int M>
+__device__ __forceinline__ void resident_bottom(const StepParams& P, const Region& R, int n_fields, int q0, const float* tab0,
+                                                int tab_step) {
+    constexpr int PITCH = resident_pitch(M);
+    const int warp = threadIdx.x >> 5, b = P.nbc;
+    const int f = warp % n_fields, part = warp / n_fields;
+    const float* tab = tab0 + f * tab_step;
+    float* p = cell_at<M>(R, q0 + f, 0, P.nz - b - 1 - R.z0);
+    const float* old = R.old + f * (b + 1) * kRW;
+    if (R.left || R.right) {
+        if (part < 3) bottom_corner<PITCH>(P, R, tab, p, old, part, 1 + f);
+    } else if (part < 2) {
+        const int col = 32 * part + (threadIdx.x & 31);
+        bottom_edge<PITCH>(P, tab, p + col, old + col, R.x0 + col < R.x1);
+    }
+}
+
+// Top band (no free surface; rows 1 .. nbc) for n_fields fields from plane q0.
+template <int M>
+__device__ __forceinline__ void resident_top(const StepParams& P, const Region& R, int n_fields, int q0, const float* tab0, int tab_step) {
+    const int b = P.nbc, nx = P.nx, r0 = nx - b - 1;
+#pragma unroll 1
+    for (int idx = threadIdx.x; idx < n_fields * b * kRW; idx += kRThreads) {
+        const int col = idx & (kRW - 1), fr = idx / kRW, f = fr / b, j = fr - f * b + 1;
+        const int i = R.x0 + col;
+        if (i >= min(R.x1, nx)) continue;
+        const float* e = R.e + (f * (b + 3) + j) * kRW + col;
+        const float* o = cell_at<M>(R, q0 + f, col, j - R.z0);
+        const float* tab = tab0 + f * tab_step;
+        auto ob = [&](int d) { return j == b ? R.e[(f * (b + 3) + b + 2) * kRW + col + d] : o[resident_pitch(M) + d]; };
+        auto wt = [&](int d) { return tab[min(min(min(i + d, nx - 1 - i - d), min(j, P.nz - 1 - j)), b + 1)]; };
+        auto topv = [&](int d) {  // top edge value of column i + d
+            return blend_edge(wt(d), e[d], edge_sum(P.qz, P.qt_z, P.qxt, e[kRW + d], o[d], ob(d)));
+        };
+        auto corner = [&](int d, float fx, int dn) {  // corner value of column i + d whose x neighbour is i + dn
+            const float sx = edge_sum(P.qx, P.qt_x, P.qxt, fx, o[d], o[dn]);
+            const float sz = edge_sum(P.qz, P.qt_z, P.qxt, e[kRW + d], o[d], ob(d));
+            return blend_corner(wt(d), e[d], sx, sz);
+        };
+        float v;
+        if (i < 1 || i > nx - 2) v = e[0];
+        else if (i <= b) v = corner(0, i + 1 <= b ? e[1] : topv(1), 1);
+        else if (i >= r0)
+            v = corner(0, !right_chunk_start(nx, b, i) ? e[-1] : (i == r0 ? topv(-1) : corner(-1, e[-2], -2)), -1);
+        else v = topv(0);
+        R.fin[idx] = v;
+    }
+    __syncthreads();
+#pragma unroll 1
+    for (int idx = threadIdx.x; idx < n_fields * b * kRW; idx += kRThreads) {
+        const int col = idx & (kRW - 1), fr = idx / kRW, f = fr / b, j = fr - f * b + 1;
+        if (R.x0 + col < min(R.x1, nx)) *cell_at<M>(R, q0 + f, col, j - R.z0) = R.fin[idx];
+    }
+}
+
+template <int M, int RT>
+__global__ void __launch_bounds__(kRThreads, 1)
+    resident_kernel(const __grid_constant__ StepParams P, const __grid_constant__ ResidentArgs A) {
+    extern __shared__ __align__(128) float smem[];
+    __shared__ int s_nrec, s_abort;
+    __shared__ float s_src[2];
+    constexpr int PITCH = resident_pitch(M), HX = resident_hx(M);
+    const ResidentLayout& L = A.L;
+    const int strip = blockIdx.x % L.strips, brow = blockIdx.x / L.strips;
+    const int b = P.nbc, nx = P.nx, nz = P.nz;
+    Region R;
+    R.x0 = L.x_edge[strip];
+    R.x1 = L.x_edge[strip + 1];
+    R.z0 = L.z_edge[brow];
+    R.z1 = L.z_edge[brow + 1];
+    R.h = R.z1 - R.z0;
+    R.left = strip == 0;
+    R.right = strip == L.strips - 1;
+    R.bottom = brow == L.rows - 1;
+    R.top = brow == 0 && !P.fs;
+    R.rim = R.left || R.right || R.z0 < M || R.z1 > nz - M;
+    const bool src_here = P.src_i >= R.x0 && P.src_i < R.x1 && P.src_j >= R.z0 && P.src_j < R.z1;
+    R.si = P.src_i - R.x0;
+    R.sj = src_here ? P.src_j - R.z0 : -1;
+    R.psize = resident_plane(M, R.h);
+    R.plane = smem;
+    float* next = smem + 5 * R.psize;
+    R.old = next;
+    if (R.bottom) next += resident_bottom_floats(b);
+    R.e = next;
+    R.fin = next + 3 * (b + 3) * kRW;
+    if (R.top) next += resident_top_floats(b);
+    float* med = next;
+    const bool med_smem = resident_smem_floats(M, b, R.h, R.bottom, R.top, true, A.iso != 0) <= (size_t)L.smem_floats;
+    if (med_smem) next += resident_med_floats(R.h, A.iso != 0);
+    int2* rec = reinterpret_cast<int2*>(next);  // receivers of the region: plane offset, number
+    next += 2 * kRRecCap;
+    R.tab = next;
+    R.src = s_src;
+
+    // ------------------------------------------------ load the region
+    if (threadIdx.x == 0) s_nrec = s_abort = 0;
+#pragma unroll 1
+    for (int d = threadIdx.x; d < 3 * (b + 2); d += kRThreads) R.tab[d] = __ldg(P.w_tab[d / (b + 2)] + d % (b + 2));
+    {
+        const int rows = R.h + 2 * M + 1, n4 = PITCH / 4;
+#pragma unroll 1
+        for (int q = 0; q < 5; ++q) {
+            const float* in = in_field(P, q);
+#pragma unroll 1
+            for (int idx = threadIdx.x; idx < rows * n4; idx += kRThreads) {
+                const int r = idx / n4, c4 = idx - r * n4;
+                const int j = R.z0 - M + r, i = R.x0 - HX + 4 * c4;
+                float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (j >= 0 && j < nz && i >= 0 && i < nx) {  // x edges and row pitch are multiples of 4
+                    v = ldg4(in + cell(P, i, j));
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) {
+                        if (i + c >= nx) set_comp(v, c, 0.f);
+                        if ((q == TXX || q == TZZ) && i + c == P.src_i && j == P.src_j) {
+                            if (src_here) s_src[q - TXX] = comp(v, c);
+                            set_comp(v, c, fadd(comp(v, c), A.wav[0]));
+                        }
+                    }
+                }
+                *reinterpret_cast<float4*>(R.plane + q * R.psize + (size_t)r * PITCH + 4 * c4) = v;
+            }
+        }
+    }
+    MedView D;
+    {
+        const size_t g = cell(P, R.x0, R.z0);
+        const float* src[7] = {A.b[0] + g, A.b[2] + g, P.lam + g, P.mu_txx + g, P.mu_txz + g, A.b[1] + g, A.b[3] + g};
+        if (med_smem) {
+            const int n = A.iso ? 5 : 7, per = R.h * (kRW / 4);
+#pragma unroll 1
+            for (int q = 0; q < n; ++q)
+#pragma unroll 1
+                for (int idx = threadIdx.x; idx < per; idx += kRThreads) {
+                    const int r = idx / (kRW / 4), c = 4 * (idx - r * (kRW / 4));
+                    const float* s = q == 0 ? src[0] : q == 1 ? src[1] : q == 2 ? src[2] : q == 3 ? src[3] : q == 4 ? src[4] : q == 5 ? src[5] : src[6];
+                    if (R.x0 + c < R.x1)
+                        *reinterpret_cast<float4*>(med + (size_t)q * R.h * kRW + r * kRW + c) = ldg4(s + (size_t)r * P.pitch + c);
+                }
+            const size_t m = (size_t)R.h * kRW;
+            D = MedView{med, A.iso ? med : med + 5 * m, med + m, A.iso ? med + m : med + 6 * m, med + 2 * m, med + 3 * m, med + 4 * m, kRW};
+        } else {
+            D = MedView{src[0], A.iso ? src[0] : src[5], src[1], A.iso ? src[1] : src[6], src[2], src[3], src[4], P.pitch};
+        }
+    }
+    __syncthreads();
+    // receivers of the region
+#pragma unroll 1
+    for (int r = threadIdx.x; r < P.n_rec; r += kRThreads) {
+        const int c = __ldg(P.rec_cell + r), j = c / P.pitch, i = c - j * P.pitch;
+        if (i >= R.x0 && i < R.x1 && j >= R.z0 && j < R.z1) {
+            const int at = atomicAdd(&s_nrec, 1);
+            if (at < kRRecCap) rec[at] = make_int2((int)((j - R.z0 + M) * PITCH + i - R.x0 + HX), r);
+        }
+    }
+    __syncthreads();
+    const int n_rec = s_nrec;
+    auto record = [&](int k) {  // receivers of step k from the planes
+        auto put = [&](int off, int r) {
+            const float* p = R.plane + off;
+            float v;
+            if (P.rec_kind == 0) v = p[VZ * R.psize];
+            else if (P.rec_kind == 1) v = p[VX * R.psize];
+            else v = fmul(fadd(p[TXX * R.psize], p[TZZ * R.psize]), 0.5f);
+            P.gather[(size_t)(k - 1) + (size_t)r * P.nt] = v;
+        };
+        if (n_rec <= kRRecCap) {
+#pragma unroll 1
+            for (int q = threadIdx.x; q < n_rec; q += kRThreads) put(rec[q].x, rec[q].y);
+        } else {  // more than the list holds: look through all of them
+#pragma unroll 1
+            for (int r = threadIdx.x; r < P.n_rec; r += kRThreads) {
+                const int c = __ldg(P.rec_cell + r), j = c / P.pitch, i = c - j * P.pitch;
+                if (i >= R.x0 && i < R.x1 && j >= R.z0 && j < R.z1) put((j - R.z0 + M) * PITCH + i - R.x0 + HX, r);
+            }
+        }
+    };
+
+    // ------------------------------------------------ exchange
+    const int box = resident_mail_items(M, L.h_max);
+    auto neighbour = [&](int dir) {
+        if (dir == 0) return R.left ? -1 : (int)blockIdx.x - 1;
+        if (dir == 1) return R.right ? -1 : (int)blockIdx.x + 1;
+        if (dir == 2) return brow == 0 ? -1 : (int)blockIdx.x - L.strips;
+        return R.bottom ? -1 : (int)blockIdx.x + L.strips;
+    };
+    const int n_items = 2 * M * R.h + 2 * M * kRW;
+    const int w = R.x1 - R.x0;
+    // kind 0: vx, vz to every side; kind 1: txx, txz to the sides, tzz, txz up and down
+    auto send = [&](int kind, uint32_t tag) {
+#pragma unroll 1
+        for (int idx = threadIdx.x; idx < n_items; idx += kRThreads) {
+            const MailItem m = resident_mail_item<M>(R.h, w, L.h_max, idx);
+            const int to = neighbour(m.dir);
+            if (to < 0 || m.col >= w) continue;
+            const int qa = kind == 0 ? VX : (m.dir < 2 ? TXX : TZZ), qb = kind == 0 ? VZ : TXZ;
+            mail_put(A.mail + (size_t)to * box + kind * (box / 2) + m.peer_slot(M, L.h_max), *cell_at<M>(R, qa, m.col, m.row),
+                     *cell_at<M>(R, qb, m.col, m.row), tag);
+        }
+    };
+    auto receive = [&](int kind, uint32_t tag) {
+        constexpr int Q = 4;
+        const ulonglong2* mine = A.mail + (size_t)blockIdx.x * box + kind * (box / 2);
+#pragma unroll 1
+        for (int base = threadIdx.x; base < n_items; base += Q * kRThreads) {
+            int slot[Q], dst[Q];
+            bool up[Q];
+            unsigned todo = 0;
+#pragma unroll
+            for (int q = 0; q < Q; ++q) {
+                const int idx = base + q * kRThreads;
+                slot[q] = dst[q] = 0;
+                up[q] = false;
+                if (idx >= n_items) continue;
+                const MailItem m = resident_mail_item<M>(R.h, w, L.h_max, idx);
+                if (neighbour(m.dir) < 0 || m.col >= w) continue;
+                slot[q] = m.slot;
+                dst[q] = (m.halo_row(M) + M) * PITCH + m.halo_col(M) + HX;
+                up[q] = m.dir >= 2;
+                todo |= 1u << q;
+            }
+#pragma unroll 1
+            for (int it = 0; todo; ++it) {
+#pragma unroll
+                for (int q = 0; q < Q; ++q)
+                    if (todo >> q & 1) {
+                        const ulonglong2 v = mail_get(mine + slot[q]);
+                        if ((uint32_t)(v.x >> 32) == tag && (uint32_t)(v.y >> 32) == tag) {
+                            const int qa = kind == 0 ? VX : (up[q] ? TZZ : TXX), qb = kind == 0 ? VZ : TXZ;
+                            R.plane[qa * R.psize + dst[q]] = __uint_as_float((uint32_t)v.x);
+                            R.plane[qb * R.psize + dst[q]] = __uint_as_float((uint32_t)v.y);
+                            todo &= ~(1u << q);
+                        }
+                    }
+                if (todo && ((it & 4095) == 4095)) {  // give up, or follow a block that has
+                    if (it >= kMailPolls || *reinterpret_cast<volatile int*>(A.status) != 0) {
+                        atomicCAS(A.status, 0, kErrResidentTimeout);
+                        s_abort = 1;
+                        todo = 0;
+                    }
+                }
+            }
+        }
+    };
+
+    // ------------------------------------------------ the steps
+    // One pass of the loop is a half step (kind 0 velocity, 1 stress), so that
+    // the code of the bands and of the exchange is there once.
+#pragma unroll 1
+    for (int hs = 0; hs < 2 * A.n_steps; ++hs) {
+        const int kind = hs & 1, s = hs >> 1;
+        if (kind == 0) resident_velocity<M, RT>(P, R, D);
+        else resident_stress<M, RT>(P, R, D);
+        __syncthreads();
+        if (R.bottom || R.top) {
+            const int nf = 2 + kind, q0 = kind ? TXX : VX, step = kind ? 0 : b + 2;
+            const float* tab = R.tab + (kind ? 2 * (b + 2) : 0);
+            if (R.bottom) resident_bottom<M>(P, R, nf, q0, tab, step);
+            if (R.top) resident_top<M>(P, R, nf, q0, tab, step);
+            __syncthreads();
+        }
+        const bool rec_now = (P.rec_kind == 2) == (kind == 1);  // vx, vz after the velocity half step, p after the stress
+        if (kind == 1) {
+            if (rec_now) record(A.k0 + s);
+            if (s + 1 == A.n_steps) break;
+            if (src_here) {  // the next step's source, before the stresses are sent
+                __syncthreads();
+                if (threadIdx.x < 2) {
+                    float* p = cell_at<M>(R, threadIdx.x == 0 ? TXX : TZZ, R.si, R.sj);
+                    s_src[threadIdx.x] = *p;
+                    *p = fadd(*p, A.wav[s + 1]);
+                }
+                __syncthreads();
+            }
+        }
+        send(kind, A.tag0 + s);
+        if (kind == 0 && rec_now) record(A.k0 + s);
+        receive(kind, A.tag0 + s);
+        __syncthreads();
+        if (s_abort) return;
+    }
+
+    // ------------------------------------------------ store the region
+#pragma unroll 1
+    for (int q = 0; q < 5; ++q) {
+        float* out = out_field(P, q);
+#pragma unroll 1
+        for (int idx = threadIdx.x; idx < R.h * (kRW / 4); idx += kRThreads) {
+            const int r = idx / (kRW / 4), c = 4 * (idx - r * (kRW / 4));
+            if (R.x0 + c < R.x1) stg4(out + cell(P, R.x0 + c, R.z0 + r), lds4(cell_at<M>(R, q, c, r)));
+        }
+    }
+}
+
+}  // namespace fomo

@@ -99,8 +99,10 @@ def set_step_kernel(mode: str = "auto", n_segs: int = 0) -> None:
     """Time-step kernels of single shots (no reference counterpart).  "split":
     four launches per step (velocity tiles, velocity band pass, stress
     tiles, stress band pass); "fused": one launch per step computing velocity
-    and stress in column strips (fails a shot it cannot run); "auto": times
-    both on the first long enough shot of a grid and keeps the faster.
+    and stress in column strips (fails a shot it cannot run); "auto": many
+    steps per launch with the fields in shared memory where the grid fits
+    (about 1.1 million padded cells), else the other two are timed on the
+    first long enough shot of a grid and the faster is kept.
     n_segs > 0 fixes the fused step's row segments per column strip.  Results
     are the same bit for bit."""
     call("fomo_b200_set_step_kernel", STEP_KERNELS[mode], int(n_segs))

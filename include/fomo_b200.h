@@ -244,22 +244,28 @@ int fomo_b200_shot_profile(uint64_t shot_handle, int32_t n_steps, FomoKernelTime
                            int32_t max_kinds, int32_t* n_kinds);
 
 /* Time-step kernel selection (no reference counterpart; a tuning control).
- * Two forms of the time step give the same bits: the split launches
- * (velocity tiles, velocity band pass, stress tiles, stress band pass) and
- * the fused step -- one launch per time step that computes velocity and
- * stress together in column strips, so every field and medium array crosses
- * HBM once (free surface, M <= 4, HABC bands that fit its first and last
- * strips).  FOMO_STEP_AUTO times both on 24 live steps each of the first
- * shot of a (grid, order, HABC width) with enough steps left, keeps the
- * faster for the process (and in the FOMO_B200_TUNE_CACHE file when that is
- * set), and runs the split launches where the fused step does not apply or
- * the shot is too short to time.  FOMO_STEP_SPLIT always runs the split
+ * Three forms of the time step give the same bits: the resident kernel --
+ * up to 256 time steps in one cooperative launch, for grids whose five
+ * fields fit the chip's shared memory (about 1.1 million padded cells; HABC
+ * bands of at most 62 layers); the split launches (velocity tiles, velocity
+ * band pass, stress tiles, stress band pass); and the fused step -- one
+ * launch per time step that computes velocity and stress together in column
+ * strips, so every field and medium array crosses HBM once (free surface,
+ * M <= 4, HABC bands that fit its first and last strips).  FOMO_STEP_AUTO
+ * runs a single shot on the resident kernel where the grid fits; elsewhere
+ * it times the other two on 24 live steps each of the first shot of a (grid,
+ * order, HABC width) with enough steps left, keeps the faster for the
+ * process (and in the FOMO_B200_TUNE_CACHE file when that is set; a grid
+ * that runs the resident kernel is entered there as not fused), and runs the
+ * split launches where the fused step does not apply or the shot is too
+ * short to time.  FOMO_STEP_SPLIT always runs the split
  * launches; FOMO_STEP_FUSED fails a single shot that the fused step does not
  * support with FOMO_EINVAL.  n_segs > 0 fixes the fused step's row segments
  * per column strip (1..64; 0 = chosen from the grid and the SM count).
  * Process-wide.  The batched and served paths run the fused step under
  * FOMO_STEP_FUSED and the split launches otherwise;
- * fomo_b200_run_shot_noalloc runs the split launches. */
+ * fomo_b200_run_shot_noalloc and fomo_b200_shot_profile run the split launches
+ * (the latter the fused step where it is selected). */
 #define FOMO_STEP_AUTO 0
 #define FOMO_STEP_SPLIT 1
 #define FOMO_STEP_FUSED 2
