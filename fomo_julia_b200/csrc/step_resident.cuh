@@ -89,72 +89,6 @@ struct Region {
     float* src;        // txx, tzz of the source cell before the source was added
 };
 
-// Side HABC of four columns x..x+3 of row j (boundary.jl:76-85) of a block on
-// one or both sides: n holds the values after the stencil update and receives
-// the final ones, o the step-start values, w the columns' weights.  All lanes
-// of the half warp that share the row call it.  edge_sum and blend_edge on
-// column pairs.
-__device__ __forceinline__ void side_rules(const StepParams& P, const Region& R, const float4& w, int x, int j, float4& n,
-                                           const float4& o) {
-    constexpr unsigned FULL = 0xffffffffu;
-    const int b = P.nbc, r0 = P.nx - b - 1;
-    const bool row = j >= (P.fs ? b : 1) && j <= P.nz - b - 2;
-    const float4 pre = n;
-    const float2 nq = make_float2(-P.qx, -P.qx), qt = make_float2(P.qt_x, P.qt_x), qxt = make_float2(P.qxt, P.qxt);
-    const float2 one = make_float2(1.f, 1.f);
-    const float2 Al = mul2(P, lo2(w), lo2(pre)), Ah = mul2(P, hi2(w), hi2(pre));
-    const float2 Wl = sub2(one, lo2(w)), Wh = sub2(one, hi2(w));
-    const float2 tl = mul2(P, qt, lo2(o)), th = mul2(P, qt, hi2(o));
-    if (R.left) {
-        const float nr = __shfl_down_sync(FULL, pre.x, 1, 16), orr = __shfl_down_sync(FULL, o.x, 1, 16);
-        const float2 sl = sub2(sub2(mul2(P, nq, make_float2(pre.y, pre.z)), tl), mul2(P, qxt, make_float2(o.y, o.z)));
-        const float2 sh = sub2(sub2(mul2(P, nq, make_float2(pre.w, nr)), th), mul2(P, qxt, make_float2(o.w, orr)));
-        const float2 fl = add2(Al, mul2(P, Wl, sl)), fh = add2(Ah, mul2(P, Wh, sh));
-        if (row && x >= 1 && x <= b) n.x = fl.x;
-        if (row && x + 1 <= b) n.y = fl.y;
-        if (row && x + 2 <= b) n.z = fh.x;
-        if (row && x + 3 <= b) n.w = fh.y;
-    }
-    if (R.right) {
-        const float nl = __shfl_up_sync(FULL, pre.w, 1, 16), ol = __shfl_up_sync(FULL, o.w, 1, 16);
-        const float2 ql = mul2(P, qxt, make_float2(ol, o.x)), qh = mul2(P, qxt, make_float2(o.y, o.z));
-        const float2 sl = sub2(sub2(mul2(P, nq, make_float2(nl, pre.x)), tl), ql);
-        const float2 sh = sub2(sub2(mul2(P, nq, make_float2(pre.y, pre.z)), th), qh);
-        float2 fl = add2(Al, mul2(P, Wl, sl)), fh = add2(Ah, mul2(P, Wh, sh));
-        // a chunk start (but the first) reads the value just computed for the column before it; the four
-        // columns hold one at most, at the same place in every lane
-        const int cs = (r0 - R.x0) & 3;
-        const float pm = __shfl_up_sync(FULL, fh.y, 1, 16);
-        const float fn = cs == 0 ? pm : cs == 1 ? fl.x : cs == 2 ? fl.y : fh.x;
-        const float t = cs == 0 ? tl.x : cs == 1 ? tl.y : cs == 2 ? th.x : th.y;
-        const float q = cs == 0 ? ql.x : cs == 1 ? ql.y : cs == 2 ? qh.x : qh.y;
-        const float A = cs == 0 ? Al.x : cs == 1 ? Al.y : cs == 2 ? Ah.x : Ah.y;
-        const float W = cs == 0 ? Wl.x : cs == 1 ? Wl.y : cs == 2 ? Wh.x : Wh.y;
-        const float f = fadd(A, fmul(W, fsub(fsub(fmul(-P.qx, fn), t), q)));
-        const int i = x + cs;
-        const bool start = i > r0 && ((i - r0) & 7) == 0;
-        if (start && cs == 0) fl.x = f;
-        if (start && cs == 1) fl.y = f;
-        if (start && cs == 2) fh.x = f;
-        if (start && cs == 3) fh.y = f;
-        if (row && x >= r0 && x <= P.nx - 2) n.x = fl.x;
-        if (row && x + 1 >= r0 && x + 1 <= P.nx - 2) n.y = fl.y;
-        if (row && x + 2 >= r0 && x + 2 <= P.nx - 2) n.z = fh.x;
-        if (row && x + 3 >= r0 && x + 3 <= P.nx - 2) n.w = fh.y;
-    }
-}
-
-// Weights of columns x..x+3 of row j from a table by distance.  Below the
-// top band they depend on the column only (every caller's row is above the
-// bottom band).
-__device__ __forceinline__ float4 side_weights(const StepParams& P, const float* tab, int x, int j) {
-    const int dj = min(j, P.nbc + 1);
-    float w[4];
-#pragma unroll
-    for (int c = 0; c < 4; ++c) w[c] = tab[max(min(min(x + c, P.nx - 1 - x - c), dj), 0)];
-    return make_float4(w[0], w[1], w[2], w[3]);
-}
-
 template <int M>
 __device__ __forceinline__ float* cell_at(const Region& R, int q, int col, int row) {
     return R.plane + q * R.psize + (size_t)(row + M) * resident_pitch(M) + col + resident_hx(M);
@@ -265,8 +199,8 @@ __device__ __forceinline__ void resident_velocity(const StepParams& P, const Reg
 #pragma unroll
             for (int rr = 0; rr < RT; ++rr) {
                 const int j = R.z0 + row + rr;
-                side_rules(P, R, side_weights(P, R.tab, x, j), x, j, nx[rr], ox[rr]);
-                side_rules(P, R, side_weights(P, R.tab + P.nbc + 2, x, j), x, j, nz[rr], oz[rr]);
+                side_rules(P, R.left, R.right, side_weights(P, R.tab, x, j), x, j, nx[rr], ox[rr]);
+                side_rules(P, R.left, R.right, side_weights(P, R.tab + P.nbc + 2, x, j), x, j, nz[rr], oz[rr]);
             }
         }
         if (on) {
@@ -374,9 +308,9 @@ __device__ __forceinline__ void resident_stress(const StepParams& P, const Regio
             for (int rr = 0; rr < RT; ++rr) {
                 const int j = R.z0 + row + rr;
                 const float4 w = side_weights(P, tab, x, j);
-                side_rules(P, R, w, x, j, n0[rr], o0[rr]);
-                side_rules(P, R, w, x, j, n1[rr], o1[rr]);
-                side_rules(P, R, w, x, j, n2[rr], o2[rr]);
+                side_rules(P, R.left, R.right, w, x, j, n0[rr], o0[rr]);
+                side_rules(P, R.left, R.right, w, x, j, n1[rr], o1[rr]);
+                side_rules(P, R.left, R.right, w, x, j, n2[rr], o2[rr]);
             }
         }
         if (on) {

@@ -18,8 +18,7 @@
 //         later); each thread owns 4 columns x 2 rows, forms
 //         x-derivatives from 128-bit shared-memory row windows and
 //         z-derivatives from a (2M+1)-row register window.  Tiles
-//         holding left/right HABC cells park their stencil values in shared
-//         memory and apply the HABC rules of step_common.cuh to them.
+//         holding left/right HABC cells apply side_rules to their registers.
 //       generic tiles (top HABC band without a free surface, or HABC bands
 //         wider than a tile allows): stencil values of the tile plus a 4 x 2
 //         margin are computed into shared memory cell by cell, then the rules.
@@ -454,13 +453,81 @@ __device__ __forceinline__ void zderiv(const StepParams& P, const float4 (&wz)[2
     }
 }
 
-// Stencil values of one tile cell, read back from shared memory by the HABC
-// rules of band tiles.
-struct TilePre {
-    const float* spre;
-    int x0, z0, f;
-    __device__ float operator()(int i, int j) const { return spre[(f * kTZ + (j - z0)) * kTX + (i - x0)]; }
-};
+// ---------------------------------------------------------------- side bands
+// Side HABC of four columns x..x+3 of row j (boundary.jl:76-85) of a tile that
+// holds the left band, the right band or both (and the columns their rules
+// read): n holds the values after the stencil update and receives the final
+// ones, o the step-start values, w the columns' weights.  The 16 lanes of a
+// half warp hold a row's 64 columns, x a multiple of 4, and all lanes of the
+// warp call it: neighbours in x come by shuffle, and edge_sum and blend_edge
+// run on column pairs.
+//
+// A tile's side cells used to go through shared memory and read step-start
+// values and weights from global memory one after another, about 15 us for
+// such a tile: one per tile row on either side, so every launch ended with
+// them.  Registers and shuffles instead: us per step, one B200, 4552 x 3927
+// 255.8 -> 217.8 (80 B a cell at the measured copy bandwidth), 3308 x 1508
+// 107.6 -> 74.6, 2108 x 908 71.4 -> 39.9, 508 x 308 52.4 -> 28.7.
+__device__ __forceinline__ void side_rules(const StepParams& P, bool left, bool right, const float4& w, int x, int j, float4& n,
+                                           const float4& o) {
+    constexpr unsigned FULL = 0xffffffffu;
+    const int b = P.nbc, r0 = P.nx - b - 1;
+    const bool row = j >= (P.fs ? b : 1) && j <= P.nz - b - 2;
+    const float4 pre = n;
+    const float2 nq = make_float2(-P.qx, -P.qx), qt = make_float2(P.qt_x, P.qt_x), qxt = make_float2(P.qxt, P.qxt);
+    const float2 one = make_float2(1.f, 1.f);
+    const float2 Al = mul2(P, lo2(w), lo2(pre)), Ah = mul2(P, hi2(w), hi2(pre));
+    const float2 Wl = sub2(one, lo2(w)), Wh = sub2(one, hi2(w));
+    const float2 tl = mul2(P, qt, lo2(o)), th = mul2(P, qt, hi2(o));
+    if (left) {
+        const float nr = __shfl_down_sync(FULL, pre.x, 1, 16), orr = __shfl_down_sync(FULL, o.x, 1, 16);
+        const float2 sl = sub2(sub2(mul2(P, nq, make_float2(pre.y, pre.z)), tl), mul2(P, qxt, make_float2(o.y, o.z)));
+        const float2 sh = sub2(sub2(mul2(P, nq, make_float2(pre.w, nr)), th), mul2(P, qxt, make_float2(o.w, orr)));
+        const float2 fl = add2(Al, mul2(P, Wl, sl)), fh = add2(Ah, mul2(P, Wh, sh));
+        if (row && x >= 1 && x <= b) n.x = fl.x;
+        if (row && x + 1 <= b) n.y = fl.y;
+        if (row && x + 2 <= b) n.z = fh.x;
+        if (row && x + 3 <= b) n.w = fh.y;
+    }
+    if (right) {
+        const float nl = __shfl_up_sync(FULL, pre.w, 1, 16), ol = __shfl_up_sync(FULL, o.w, 1, 16);
+        const float2 ql = mul2(P, qxt, make_float2(ol, o.x)), qh = mul2(P, qxt, make_float2(o.y, o.z));
+        const float2 sl = sub2(sub2(mul2(P, nq, make_float2(nl, pre.x)), tl), ql);
+        const float2 sh = sub2(sub2(mul2(P, nq, make_float2(pre.y, pre.z)), th), qh);
+        float2 fl = add2(Al, mul2(P, Wl, sl)), fh = add2(Ah, mul2(P, Wh, sh));
+        // a chunk start (but the first) reads the value just computed for the column before it; the four
+        // columns hold one at most, at the same place in every lane (x is a multiple of 4)
+        const int cs = (r0 - x) & 3;
+        const float pm = __shfl_up_sync(FULL, fh.y, 1, 16);
+        const float fn = cs == 0 ? pm : cs == 1 ? fl.x : cs == 2 ? fl.y : fh.x;
+        const float t = cs == 0 ? tl.x : cs == 1 ? tl.y : cs == 2 ? th.x : th.y;
+        const float q = cs == 0 ? ql.x : cs == 1 ? ql.y : cs == 2 ? qh.x : qh.y;
+        const float A = cs == 0 ? Al.x : cs == 1 ? Al.y : cs == 2 ? Ah.x : Ah.y;
+        const float W = cs == 0 ? Wl.x : cs == 1 ? Wl.y : cs == 2 ? Wh.x : Wh.y;
+        const float f = fadd(A, fmul(W, fsub(fsub(fmul(-P.qx, fn), t), q)));
+        const int i = x + cs;
+        const bool start = i > r0 && ((i - r0) & 7) == 0;
+        if (start && cs == 0) fl.x = f;
+        if (start && cs == 1) fl.y = f;
+        if (start && cs == 2) fh.x = f;
+        if (start && cs == 3) fh.y = f;
+        if (row && x >= r0 && x <= P.nx - 2) n.x = fl.x;
+        if (row && x + 1 >= r0 && x + 1 <= P.nx - 2) n.y = fl.y;
+        if (row && x + 2 >= r0 && x + 2 <= P.nx - 2) n.z = fh.x;
+        if (row && x + 3 >= r0 && x + 3 <= P.nx - 2) n.w = fh.y;
+    }
+}
+
+// Weights of columns x..x+3 of row j from a table by distance.  Below the
+// top band they depend on the column only (every caller's row is above the
+// bottom band).
+__device__ __forceinline__ float4 side_weights(const StepParams& P, const float* tab, int x, int j) {
+    const int dj = min(j, P.nbc + 1);
+    float w[4];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) w[c] = tab[max(min(min(x + c, P.nx - 1 - x - c), dj), 0)];
+    return make_float4(w[0], w[1], w[2], w[3]);
+}
 
 // L2 prefetch of the boxes of tile `tile` when it is a fast tile of this
 // launch (defined after classify).  The single-shot fast tiles pass
@@ -582,26 +649,14 @@ __device__ __forceinline__ void fast_vel(const StepParams& P, const TiledArgs& T
                 }
         }
     }
-    if (band) {
-        __syncthreads();  // every thread is done with the boxes
-        float* spre = smem;  // [2][kTZ][kTX]
+    if (band) {  // block-uniform: every lane takes part
+        const bool left = x0 <= P.nbc, right = x0 + kTX - 1 >= P.nx - P.nbc - 1;
 #pragma unroll
         for (int rr = 0; rr < 2; ++rr) {
-            const int po = (2 * rp + rr) * kTX + xr;
-            *reinterpret_cast<float4*>(spre + po) = ox[rr];
-            *reinterpret_cast<float4*>(spre + kPBox + po) = oz[rr];
+            const int po = (2 * rp + rr) * kTX + xr, j = zt + rr;
+            side_rules(P, left, right, side_weights(P, P.w_tab[0], x, j), x, j, ox[rr], lds4(p_vx + po));
+            side_rules(P, left, right, side_weights(P, P.w_tab[1], x, j), x, j, oz[rr], lds4(p_vz + po));
         }
-        __syncthreads();
-        const HabcPoint<TilePre> hx{P, TilePre{spre, x0, z0, 0}, P.in[VX], P.w_tab[0]};
-        const HabcPoint<TilePre> hz{P, TilePre{spre, x0, z0, 1}, P.in[VZ], P.w_tab[1]};
-#pragma unroll
-        for (int rr = 0; rr < 2; ++rr)
-#pragma unroll
-            for (int c = 0; c < 4; ++c)
-                if (x + c < x_end && row_stored(P, zt + rr) && lr_band_cell(P, x + c, zt + rr)) {
-                    set_comp(ox[rr], c, hx.final_value(x + c, zt + rr));
-                    set_comp(oz[rr], c, hz.final_value(x + c, zt + rr));
-                }
     }
     if (x < x_end) {
 #pragma unroll
@@ -715,29 +770,16 @@ __device__ __forceinline__ void fast_str(const StepParams& P, const TiledArgs& T
                 }
         }
     }
-    if (band) {
-        __syncthreads();
-        float* spre = smem;  // [3][kTZ][kTX]
+    if (band) {  // the step-start values are the boxes', before the source
+        const bool left = x0 <= P.nbc, right = x0 + kTX - 1 >= P.nx - P.nbc - 1;
 #pragma unroll
         for (int rr = 0; rr < 2; ++rr) {
-            const int po = (2 * rp + rr) * kTX + xr;
-            *reinterpret_cast<float4*>(spre + po) = oxx[rr];
-            *reinterpret_cast<float4*>(spre + kPBox + po) = ozz[rr];
-            *reinterpret_cast<float4*>(spre + 2 * kPBox + po) = oxz[rr];
+            const int po = (2 * rp + rr) * kTX + xr, j = zt + rr;
+            const float4 w = side_weights(P, P.w_tab[2], x, j);
+            side_rules(P, left, right, w, x, j, oxx[rr], lds4(p_xx + po));
+            side_rules(P, left, right, w, x, j, ozz[rr], lds4(p_zz + po));
+            side_rules(P, left, right, w, x, j, oxz[rr], lds4(p_xz + po));
         }
-        __syncthreads();
-        const HabcPoint<TilePre> h0{P, TilePre{spre, x0, z0, 0}, P.in[TXX], P.w_tab[2]};
-        const HabcPoint<TilePre> h1{P, TilePre{spre, x0, z0, 1}, P.in[TZZ], P.w_tab[2]};
-        const HabcPoint<TilePre> h2{P, TilePre{spre, x0, z0, 2}, P.in[TXZ], P.w_tab[2]};
-#pragma unroll
-        for (int rr = 0; rr < 2; ++rr)
-#pragma unroll
-            for (int c = 0; c < 4; ++c)
-                if (x + c < x_end && row_stored(P, zt + rr) && lr_band_cell(P, x + c, zt + rr)) {
-                    set_comp(oxx[rr], c, h0.final_value(x + c, zt + rr));
-                    set_comp(ozz[rr], c, h1.final_value(x + c, zt + rr));
-                    set_comp(oxz[rr], c, h2.final_value(x + c, zt + rr));
-                }
     }
     if (x < x_end) {
 #pragma unroll
