@@ -53,14 +53,15 @@ __host__ __device__ constexpr int resident_pitch(int M) { return kRW + 2 * resid
 __host__ __device__ constexpr int resident_mail_items(int M, int h_max) { return 2 * (2 * M * h_max + 2 * M * kRW); }
 
 // Shared-memory floats of a region of h rows: five field planes, the bottom
-// band's scratch (step-start values of its b rows and the row above), the top
+// band's scratch (step-start values of its b rows and the row above; x terms of
+// the corners), the top
 // band's (no free surface: values before the band rule of rows 0..b+1, one
 // row of step-start values; results), the weight tables, the receiver list
 // and a few words.
 __host__ __device__ constexpr size_t resident_plane(int M, int h) { return (size_t)(h + 2 * M + 1) * resident_pitch(M); }
-__host__ __device__ constexpr size_t resident_bottom_floats(int b) { return (size_t)3 * (b + 1) * kRW; }
+__host__ __device__ constexpr size_t resident_bottom_floats(int b) { return (size_t)3 * (2 * b + 1) * kRW; }
 __host__ __device__ constexpr size_t resident_top_floats(int b) { return (size_t)3 * (2 * b + 3) * kRW; }
-__host__ __device__ constexpr size_t resident_tail_floats(int b) { return (size_t)3 * (b + 2) + 2 * kRRecCap + 16; }
+__host__ __device__ constexpr size_t resident_tail_floats(int b) { return (size_t)3 * kRW + 3 * (b + 2) + 2 * kRRecCap + 16; }
 __host__ __device__ constexpr size_t resident_med_floats(int h, bool iso) { return (size_t)(iso ? 5 : 7) * h * kRW; }
 __host__ __device__ constexpr size_t resident_smem_floats(int M, int b, int h, bool bottom, bool top, bool med, bool iso) {
     return 5 * resident_plane(M, h) + (bottom ? resident_bottom_floats(b) : 0) + (top ? resident_top_floats(b) : 0) +

@@ -83,9 +83,10 @@ struct Region {
     int si, sj;        // source, in region coordinates; sj < 0: not here
     float* plane;      // five planes of `psize` floats, row pitch PITCH, cell (x0, z0) at M rows + HX columns
     size_t psize;
-    float* old;        // bottom band: step-start values [3][b+1][kRW], row 0 the row above the band
+    float *old, *sx;   // bottom band: step-start values [3][b+1][kRW], row 0 the row above the band; x terms [3][b][kRW]
     float *e, *fin;    // top band: [3][b+3][kRW] (row b+2: step-start values of row b+1), [3][b][kRW]
     float* tab;        // weights of vx, vz, tau by distance, b + 2 each
+    float* wcol;       // and of the region's columns, kRW each (rows below the top band)
     float* src;        // txx, tzz of the source cell before the source was added
 };
 
@@ -97,27 +98,72 @@ __device__ __forceinline__ float* cell_at(const Region& R, int q, int col, int r
 // Where a row's values go after the side rules.
 __device__ __forceinline__ bool in_top_rows(const StepParams& P, int j) { return !P.fs && j >= 1 && j <= P.nbc; }
 
-// Stores four columns of field f (of the half step; plane q) of row j: to the
-// plane, with the step-start values of the rows the bottom recurrence reads
-// beside; rows of the top band to its scratch, their plane keeps the
-// step-start values.
+// Weights of columns x..x+3 of row j from table `t` (0 vx, 1 vz, 2 tau), every
+// row above the bottom band: below the top band they depend on the column
+// only and come as one 16-byte load.
+__device__ __forceinline__ float4 region_weights(const StepParams& P, const Region& R, int t, int x, int j) {
+    if (P.fs || j > P.nbc) return lds4(R.wcol + t * kRW + (x - R.x0));
+    return side_weights(P, R.tab + t * (P.nbc + 2), x, j);
+}
+
+// Four columns of a row of the bottom band (row jb of field f): the values
+// before the HABC go to the plane, the step-start values to R.old and, in a
+// block at a corner, the x terms of the corner columns to R.sx (side_rules'
+// sums; other columns hold whatever comes out).  All lanes of the half warp
+// that share the row call it.
+__device__ __forceinline__ void put_band_row(const StepParams& P, const Region& R, int f, float* p, int col, int jb,
+                                             const float4& n, const float4& o, bool on) {
+    constexpr unsigned FULL = 0xffffffffu;
+    const int b = P.nbc;
+    if (R.left || R.right) {
+        const float2 nq = make_float2(-P.qx, -P.qx), qt = make_float2(P.qt_x, P.qt_x), qxt = make_float2(P.qxt, P.qxt);
+        const float2 tl = mul2(P, qt, lo2(o)), th = mul2(P, qt, hi2(o));
+        float2 nl, nh, ol, oh;  // the neighbours towards the interior: i+1 on the left, i-1 on the right
+        const bool l = R.left && R.x0 + col <= b;  // a block on both sides: by group of columns
+        const float nu = __shfl_up_sync(FULL, n.w, 1, 16), ou = __shfl_up_sync(FULL, o.w, 1, 16);
+        const float nd = __shfl_down_sync(FULL, n.x, 1, 16), od = __shfl_down_sync(FULL, o.x, 1, 16);
+        if (l) {
+            nl = make_float2(n.y, n.z), nh = make_float2(n.w, nd);
+            ol = make_float2(o.y, o.z), oh = make_float2(o.w, od);
+        } else {
+            nl = make_float2(nu, n.x), nh = make_float2(n.y, n.z);
+            ol = make_float2(ou, o.x), oh = make_float2(o.y, o.z);
+        }
+        const float2 sl = sub2(sub2(mul2(P, nq, nl), tl), mul2(P, qxt, ol));
+        const float2 sh = sub2(sub2(mul2(P, nq, nh), th), mul2(P, qxt, oh));
+        if (on) *reinterpret_cast<float4*>(R.sx + (f * b + jb) * kRW + col) = make_float4(sl.x, sl.y, sh.x, sh.y);
+    }
+    if (on) {
+        *reinterpret_cast<float4*>(p) = n;
+        *reinterpret_cast<float4*>(R.old + (f * (b + 1) + jb + 1) * kRW + col) = o;
+    }
+}
+
+// Stores four columns of field f (of the half step; plane q) of row j above
+// the bottom band: to the plane; rows of the top band to its scratch, their
+// plane keeps the step-start values.
 template <int M>
 __device__ __forceinline__ void put_row(const StepParams& P, const Region& R, int f, int q, int col, int row, const float4& n,
                                         const float4& o, bool zero, bool src_row) {
-    const int b = P.nbc, j = R.z0 + row, jb = j - (P.nz - b - 1);
+    const int b = P.nbc, j = R.z0 + row;
     float* p = cell_at<M>(R, q, col, row);
-    if (in_top_rows(P, j)) {
-        *reinterpret_cast<float4*>(R.e + (f * (b + 3) + j) * kRW + col) = n;
-        if (src_row) *reinterpret_cast<float4*>(p) = o;  // the band rule reads step-start values here
-        return;
+    if (R.top) {
+        if (in_top_rows(P, j)) {
+            *reinterpret_cast<float4*>(R.e + (f * (b + 3) + j) * kRW + col) = n;
+            if (src_row) *reinterpret_cast<float4*>(p) = o;  // the band rule reads step-start values here
+            return;
+        }
+        if (j == b + 1) {
+            *reinterpret_cast<float4*>(R.e + (f * (b + 3) + b + 1) * kRW + col) = n;
+            *reinterpret_cast<float4*>(R.e + (f * (b + 3) + b + 2) * kRW + col) = o;
+        }
     }
-    if (jb >= -1 && jb < b) *reinterpret_cast<float4*>(R.old + (f * (b + 1) + jb + 1) * kRW + col) = o;
-    if (R.top && j == b + 1) {
-        *reinterpret_cast<float4*>(R.e + (f * (b + 3) + b + 1) * kRW + col) = n;
-        *reinterpret_cast<float4*>(R.e + (f * (b + 3) + b + 2) * kRW + col) = o;
-    }
+    if (R.bottom && j == P.nz - b - 2) *reinterpret_cast<float4*>(R.old + f * (b + 1) * kRW + col) = o;
     *reinterpret_cast<float4*>(p) = zero ? make_float4(0.f, 0.f, 0.f, 0.f) : n;
 }
+
+// Whether a warp's rows j .. j+n-1 hold rows of the bottom band.
+__device__ __forceinline__ bool band_rows(const StepParams& P, int j, int n) { return j + n > P.nz - P.nbc - 1 && j <= P.nz - 2; }
 
 // Medium of the region: global memory or its copy in shared memory.
 struct MedView {
@@ -199,17 +245,24 @@ __device__ __forceinline__ void resident_velocity(const StepParams& P, const Reg
 #pragma unroll
             for (int rr = 0; rr < RT; ++rr) {
                 const int j = R.z0 + row + rr;
-                side_rules(P, R.left, R.right, side_weights(P, R.tab, x, j), x, j, nx[rr], ox[rr]);
-                side_rules(P, R.left, R.right, side_weights(P, R.tab + P.nbc + 2, x, j), x, j, nz[rr], oz[rr]);
+                side_rules(P, R.left, R.right, region_weights(P, R, 0, x, j), x, j, nx[rr], ox[rr]);
+                side_rules(P, R.left, R.right, region_weights(P, R, 1, x, j), x, j, nz[rr], oz[rr]);
             }
         }
-        if (on) {
+        const bool band = R.bottom && band_rows(P, R.z0 + base + (threadIdx.x >> 5) * 2 * RT, 2 * RT);
 #pragma unroll
-            for (int rr = 0; rr < RT; ++rr)
-                if (row + rr < R.h) {
-                    put_row<M>(P, R, 0, VX, col, row + rr, nx[rr], ox[rr], false, false);
-                    put_row<M>(P, R, 1, VZ, col, row + rr, nz[rr], oz[rr], false, false);
-                }
+        for (int rr = 0; rr < RT; ++rr) {
+            const int jb = R.z0 + row + rr - (P.nz - P.nbc - 1);
+            const bool here = on && row + rr < R.h, in_band = jb >= 0 && jb < P.nbc;
+            if (band) {
+                const int jc = min(max(jb, 0), P.nbc - 1);
+                put_band_row(P, R, 0, cell_at<M>(R, VX, col, row + rr), col, jc, nx[rr], ox[rr], here && in_band);
+                put_band_row(P, R, 1, cell_at<M>(R, VZ, col, row + rr), col, jc, nz[rr], oz[rr], here && in_band);
+            }
+            if (here && !in_band) {
+                put_row<M>(P, R, 0, VX, col, row + rr, nx[rr], ox[rr], false, false);
+                put_row<M>(P, R, 1, VZ, col, row + rr, nz[rr], oz[rr], false, false);
+            }
         }
     }
 }
@@ -303,147 +356,157 @@ __device__ __forceinline__ void resident_stress(const StepParams& P, const Regio
         }
         if ((R.left || R.right) && side_rows(P, R.z0 + base + (threadIdx.x >> 5) * 2 * RT, 2 * RT)) {
             __syncwarp();
-            const float* tab = R.tab + 2 * (P.nbc + 2);
 #pragma unroll
             for (int rr = 0; rr < RT; ++rr) {
                 const int j = R.z0 + row + rr;
-                const float4 w = side_weights(P, tab, x, j);
+                const float4 w = region_weights(P, R, 2, x, j);
                 side_rules(P, R.left, R.right, w, x, j, n0[rr], o0[rr]);
                 side_rules(P, R.left, R.right, w, x, j, n1[rr], o1[rr]);
                 side_rules(P, R.left, R.right, w, x, j, n2[rr], o2[rr]);
             }
         }
-        if (on) {
+        const bool band = R.bottom && band_rows(P, R.z0 + base + (threadIdx.x >> 5) * 2 * RT, 2 * RT);
 #pragma unroll
-            for (int rr = 0; rr < RT; ++rr)
-                if (row + rr < R.h) {
-                    const bool zero = in_free_surface_rows(P, R.z0 + row + rr);
-                    const bool src = row + rr == R.sj && R.si >= col && R.si < col + 4;
-                    put_row<M>(P, R, 0, TXX, col, row + rr, n0[rr], o0[rr], false, src);
-                    put_row<M>(P, R, 1, TZZ, col, row + rr, n1[rr], o1[rr], zero, src);
-                    put_row<M>(P, R, 2, TXZ, col, row + rr, n2[rr], o2[rr], zero, false);
-                }
+        for (int rr = 0; rr < RT; ++rr) {
+            const int jb = R.z0 + row + rr - (P.nz - P.nbc - 1);
+            const bool here = on && row + rr < R.h, in_band = jb >= 0 && jb < P.nbc;
+            if (band) {
+                const int jc = min(max(jb, 0), P.nbc - 1);
+                put_band_row(P, R, 0, cell_at<M>(R, TXX, col, row + rr), col, jc, n0[rr], o0[rr], here && in_band);
+                put_band_row(P, R, 1, cell_at<M>(R, TZZ, col, row + rr), col, jc, n1[rr], o1[rr], here && in_band);
+                put_band_row(P, R, 2, cell_at<M>(R, TXZ, col, row + rr), col, jc, n2[rr], o2[rr], here && in_band);
+            }
+            if (here && !in_band) {
+                const bool zero = in_free_surface_rows(P, R.z0 + row + rr);
+                const bool src = row + rr == R.sj && R.si >= col && R.si < col + 4;
+                put_row<M>(P, R, 0, TXX, col, row + rr, n0[rr], o0[rr], false, src);
+                put_row<M>(P, R, 1, TZZ, col, row + rr, n1[rr], o1[rr], zero, src);
+                put_row<M>(P, R, 2, TXZ, col, row + rr, n2[rr], o2[rr], zero, false);
+            }
         }
     }
 }
 
-// One warp's part of the bottom band's recurrence along j (rows nz-nbc-1 ..
-// nz-2) of one field, a column per lane.  `p` is the lane's column of the plane
-// at the first band row: values after the stencil update, replaced by the
-// final ones; `old` the column's step-start values, row 0 being the row above
-// the band.  A column's chain needs its own column only: five dependent
-// operations a row; loads and everything off the chain run G rows ahead.
-constexpr int kBandGroup = 5;
-template <int PITCH>
-__device__ __forceinline__ void bottom_edge(const StepParams& P, const float* tab, float* p, const float* old, bool store) {
-    constexpr int G = kBandGroup;
-    const int b = P.nbc;
-    float fp = p[-PITCH], op = old[0];
-    auto rows = [&](int g, int n) {
-        float A[G], W[G], t1[G], t2[G];
-        float* pg = p + g * PITCH;
-        const float *og = old + (g + 1) * kRW, *wg = tab + b - g;  // distance nz - 1 - j = b - jb
-#pragma unroll
-        for (int r = 0; r < G; ++r)
-            if (r < n) {
-                const float w = wg[-r], ov = og[r * kRW];
-                A[r] = fmul(w, pg[r * PITCH]);
-                W[r] = fsub(1.f, w);
-                t1[r] = fmul(P.qt_z, ov);
-                t2[r] = fmul(P.qxt, op);
-                op = ov;
-            }
-#pragma unroll
-        for (int r = 0; r < G; ++r)
-            if (r < n) {
-                fp = fadd(A[r], fmul(W[r], fsub(fsub(fmul(-P.qz, fp), t1[r]), t2[r])));
-                if (store) pg[r * PITCH] = fp;
-            }
-    };
-    int g = 0;
-#pragma unroll 1
-    for (; g + G <= b; g += G) rows(g, G);
-#pragma unroll 1
-    for (; g < b; ++g) rows(g, 1);
-}
+// Bottom band (rows nz-nbc-1 .. nz-2) of the block's columns for n_fields
+// fields from plane q0: the recurrence band_march runs,
+//   f = A + W (sx + ((-qz f' - qt_z ov) - qxt ov')),  A = w pv,
+// a column per lane, in the plane itself; put_band_row left pv in the plane, ov
+// in R.old (row 0: the row above the band) and sx in R.sx, so a column reads
+// its own values only.  A few warps alone on their SM run at the latency of
+// what they wait for and at one instruction a cycle at best, so a row is kept
+// to its loads, four or five products and the chain of six operations, with the
+// next four rows loaded ahead of it (past the band's end too: shared memory
+// follows).  In a block at a corner one more warp holds the columns of all
+// fields that read their neighbour's final value (the last bottom-left column
+// and the bottom-right chunk starts), kBandStage rows behind the others.
+// Cycles for 50 rows of three fields on one SM: neighbours by shuffle inside
+// the chain 13,900 at a corner and 3,300 on the edge; x terms read from the
+// plane by two warps that meet once a group 8,250; this form 5,100 and 3,000.
+constexpr int kBandStage = 8;
 
-// The same near a corner, where f = A + W (sx + sz): W = (1 - w) / 2 and sx the
-// x term in a corner column, W = 1 - w and sx = -0 (which adds nothing) in an
-// edge column.  Three warps (`part`) share a field: two march the columns that
-// read their neighbour's value before the HABC, the third, one group of rows
-// behind, the columns that read its final value (the last bottom-left column
-// and the bottom-right chunk starts).  They meet at named barrier `bar` once a
-// group: every value of its rows is read before any is replaced.
-template <int PITCH>
-__device__ __forceinline__ void bottom_corner(const StepParams& P, const Region& R, const float* tab, float* p0,
-                                              const float* old0, int part, int bar) {
-    constexpr int G = kBandGroup;
-    const int lane = threadIdx.x & 31, b = P.nbc, nx = P.nx, r0 = nx - b - 1;
-    const int nr = R.right ? (b + 7) / 8 : 0;
-    const bool second = part == 2;
-    int i = second ? (lane < nr ? r0 + 8 * lane : b) : R.x0 + 32 * part + lane;
-    bool store = second ? lane < nr + (R.left ? 1 : 0) : i < min(R.x1, nx);
-    if (!store) i = R.x0;
-    const bool rim = i <= 0 || i >= nx - 1;
-    const bool lc = i >= 1 && i <= b, rc = i >= r0 && i <= nx - 2, corner = lc || rc;
-    const bool redo = (lc && i == b) || (rc && right_chunk_start(nx, b, i));
-    if (!second && redo) store = false;
-    const int dx = max(min(min(i, nx - 1 - i), b + 1), 0), dn = lc ? 1 : (rc ? -1 : 0);
-    const float h = corner ? 0.5f : 1.f;
-    float* p = p0 + (i - R.x0);
-    const float* old = old0 + (i - R.x0);
-    float fp = p[-PITCH], op = old[0];
-    auto sync = [&] { asm volatile("bar.sync %0, 96;" ::"r"(bar) : "memory"); };
-    auto rows = [&](int g, int n) {
-        float A[G], W[G], t1[G], t2[G], sx[G];
-        float* pg = p + g * PITCH;
-        const float* og = old + (g + 1) * kRW;
+struct BandRows {  // four rows as loaded
+    float pv[4], ov[4], w[4], s[4];
+};
+
+// KIND 0: edge columns only; 1: near a corner; 2: columns that read their
+// neighbour's final value (dn columns away).
+template <int PITCH, int KIND>
+struct BandMarch {
+    const StepParams& P;
+    const float* tab;
+    float* p;
+    const float *old, *sx;
+    int dx, dn;
+    float h;
+    bool corner, store;
+    float fp, op;
+
+    __device__ __forceinline__ void load(BandRows& o, int j) const {
 #pragma unroll
-        for (int r = 0; r < G; ++r)
-            if (r < n) {
-                const float w = tab[min(dx, b - g - r)], ov = og[r * kRW], pv = pg[r * PITCH];
-                const float s = edge_sum(P.qx, P.qt_x, P.qxt, pg[r * PITCH + dn], ov, og[r * kRW + dn]);
-                sx[r] = corner ? s : -0.f;
-                A[r] = rim ? pv : fmul(w, pv);
-                W[r] = fmul(fsub(1.f, w), h);
-                t1[r] = fmul(P.qt_z, ov);
-                t2[r] = fmul(P.qxt, op);
-                op = ov;
-            }
-        if (!second) sync();
-#pragma unroll
-        for (int r = 0; r < G; ++r)
-            if (r < n) {
-                const float f = fadd(A[r], fmul(W[r], fadd(sx[r], fsub(fsub(fmul(-P.qz, fp), t1[r]), t2[r]))));
-                fp = rim ? A[r] : f;  // the grid's rim keeps its value
-                if (store) pg[r * PITCH] = fp;
-            }
-    };
-    if (second) sync();  // the first group has been read
-    int g = 0;
-#pragma unroll 1
-    for (; g < b; g += G) {
-        if (second) sync();  // the group is final but for this warp's columns
-        rows(g, min(G, b - g));
+        for (int r = 0; r < 4; ++r) {
+            o.pv[r] = p[(j + r) * PITCH];
+            o.ov[r] = old[(j + r + 1) * kRW];
+            o.w[r] = tab[KIND ? min(dx, P.nbc - j - r) : P.nbc - j - r];
+            if (KIND == 1) o.s[r] = corner ? sx[(j + r) * kRW] : -0.f;
+            if (KIND == 2) o.s[r] = fmul(P.qxt, old[(j + r + 1) * kRW + dn]);
+        }
     }
-    if (!second) sync();
-}
+    // KIND 2: the x terms, from the neighbour's final values
+    __device__ __forceinline__ void finals(BandRows& o, int j) const {
+#pragma unroll
+        for (int r = 0; r < 4; ++r)
+            o.s[r] = fsub(fsub(fmul(-P.qx, p[(j + r) * PITCH + dn]), fmul(P.qt_x, o.ov[r])), o.s[r]);
+    }
+    __device__ __forceinline__ void march(const BandRows& o, int j) {
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            const float A = fmul(o.w[r], o.pv[r]), w1 = fsub(1.f, o.w[r]), W = KIND ? fmul(w1, h) : w1;
+            const float z = fsub(fsub(fmul(-P.qz, fp), fmul(P.qt_z, o.ov[r])), fmul(P.qxt, op));
+            op = o.ov[r];
+            fp = fadd(A, fmul(W, KIND ? fadd(o.s[r], z) : z));
+            if (store && j + r < P.nbc) p[(j + r) * PITCH] = fp;
+        }
+    }
+};
 
-// Bottom band of the block's columns for n_fields fields from plane q0.
 template <int M>
 __device__ __forceinline__ void resident_bottom(const StepParams& P, const Region& R, int n_fields, int q0, const float* tab0,
                                                 int tab_step) {
     constexpr int PITCH = resident_pitch(M);
-    const int warp = threadIdx.x >> 5, b = P.nbc;
-    const int f = warp % n_fields, part = warp / n_fields;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, b = P.nbc, nx = P.nx, r0 = nx - b - 1;
+    const bool corners = R.left || R.right, second = corners && warp == 2 * n_fields;
+    if (warp >= 2 * n_fields && !second) return;
+    // the lane's column: of the region, or of the columns that read a final value (at most 9 a field)
+    const int nr = R.right ? (b + 7) / 8 : 0, per = nr + (R.left ? 1 : 0);
+    const int f = second ? min(lane / per, n_fields - 1) : warp >> 1, c = lane - f * per;
+    const int i = !second ? R.x0 + 32 * (warp & 1) + lane : lane >= per * n_fields ? R.x0 + 1 : c < nr ? r0 + 8 * c : b;
+    const int col = i - R.x0;
+    const bool lc = i >= 1 && i <= b, rc = i >= r0 && i <= nx - 2;
+    const bool redo = (lc && i == b) || (rc && right_chunk_start(nx, b, i));
     const float* tab = tab0 + f * tab_step;
-    float* p = cell_at<M>(R, q0 + f, 0, P.nz - b - 1 - R.z0);
-    const float* old = R.old + f * (b + 1) * kRW;
-    if (R.left || R.right) {
-        if (part < 3) bottom_corner<PITCH>(P, R, tab, p, old, part, 1 + f);
-    } else if (part < 2) {
-        const int col = 32 * part + (threadIdx.x & 31);
-        bottom_edge<PITCH>(P, tab, p + col, old + col, R.x0 + col < R.x1);
+    float* p = cell_at<M>(R, q0 + f, col, P.nz - b - 1 - R.z0);
+    const float* old = R.old + f * (b + 1) * kRW + col;
+    const float *sx = R.sx + f * b * kRW + col;
+    const int dx = max(min(min(i, nx - 1 - i), b + 1), 0);
+    const float h = lc || rc ? 0.5f : 1.f;
+    BandRows X, Y;
+    if (!corners) {
+        BandMarch<PITCH, 0> B{P, tab, p, old, sx, dx, 0, h, false, i < R.x1, p[-PITCH], old[0]};
+        B.load(X, 0);
+#pragma unroll 1
+        for (int j = 0; j < b; j += 8) {
+            B.load(Y, j + 4);
+            B.march(X, j);
+            B.load(X, j + 8);
+            B.march(Y, j + 4);
+        }
+        return;
+    }
+    auto sync = [&] { asm volatile("bar.sync 1, %0;" ::"r"(32 * (2 * n_fields + 1)) : "memory"); };
+    static_assert(kBandStage == 8, "two groups of four rows");
+    if (!second) {
+        BandMarch<PITCH, 1> B{P, tab, p, old, sx, dx, 0, h, lc || rc, i < min(R.x1, nx - 1) && i >= 1 && !redo, p[-PITCH], old[0]};
+        B.load(X, 0);
+#pragma unroll 1
+        for (int j = 0; j < b; j += kBandStage) {
+            B.load(Y, j + 4);
+            B.march(X, j);
+            B.load(X, j + 8);
+            B.march(Y, j + 4);
+            sync();
+        }
+    } else {
+        BandMarch<PITCH, 2> B{P, tab, p, old, sx, dx, lc ? 1 : -1, h, true, lane < per * n_fields, p[-PITCH], old[0]};
+#pragma unroll 1
+        for (int j = 0; j < b; j += kBandStage) {
+            sync();
+            B.load(X, j);
+            B.load(Y, j + 4);
+            B.finals(X, j);
+            B.finals(Y, j + 4);
+            B.march(X, j);
+            B.march(Y, j + 4);
+        }
     }
 }
 
@@ -513,6 +576,7 @@ __global__ void __launch_bounds__(kRThreads, 1)
     R.plane = smem;
     float* next = smem + 5 * R.psize;
     R.old = next;
+    R.sx = next + 3 * (b + 1) * kRW;
     if (R.bottom) next += resident_bottom_floats(b);
     R.e = next;
     R.fin = next + 3 * (b + 3) * kRW;
@@ -522,13 +586,19 @@ __global__ void __launch_bounds__(kRThreads, 1)
     if (med_smem) next += resident_med_floats(R.h, A.iso != 0);
     int2* rec = reinterpret_cast<int2*>(next);  // receivers of the region: plane offset, number
     next += 2 * kRRecCap;
+    R.wcol = next;
+    next += 3 * kRW;
     R.tab = next;
     R.src = s_src;
 
     // ------------------------------------------------ load the region
     if (threadIdx.x == 0) s_nrec = s_abort = 0;
 #pragma unroll 1
-    for (int d = threadIdx.x; d < 3 * (b + 2); d += kRThreads) R.tab[d] = __ldg(P.w_tab[d / (b + 2)] + d % (b + 2));
+    for (int d = threadIdx.x; d < 3 * (b + 2); d += kRThreads) R.tab[d] = __ldg(w_table(P, d / (b + 2)) + d % (b + 2));
+    if (threadIdx.x < 3 * kRW) {
+        const int i = R.x0 + (threadIdx.x & (kRW - 1));
+        R.wcol[threadIdx.x] = __ldg(w_table(P, threadIdx.x / kRW) + max(min(min(i, nx - 1 - i), b + 1), 0));
+    }
     {
         const int rows = R.h + 2 * M + 1, n4 = PITCH / 4;
 #pragma unroll 1

@@ -45,8 +45,9 @@ constexpr int kTileBlocks = 5;
 constexpr int kStripW = 28;     // columns a band-pass warp stores
 constexpr int kMarchRows = 16;  // band rows staged per chunk by the band pass
 
-// Band-pass strips over a grid nx cells wide.
-__host__ __device__ constexpr int band_block_count(int nx) { return (nx + kStripW - 1) / kStripW; }
+// Band-pass strips over a grid nx cells wide (strip s stores columns
+// s * kStripW - 2 .. + kStripW - 1).
+__host__ __device__ constexpr int band_block_count(int nx) { return (nx + 2 + kStripW - 1) / kStripW; }
 constexpr int kEdgeX = 4, kEdgeZ = 2;  // margin of stencil values around an edge tile
 
 template <int M>
@@ -187,11 +188,6 @@ __device__ __forceinline__ void tma_prefetch_2d(const CUtensorMap* map, int x, i
                  : "memory");
 }
 
-// 4-byte asynchronous global -> shared copy; valid == false writes zero.
-__device__ __forceinline__ void cp_async4(float* dst, const float* src, bool valid) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(valid ? 4 : 0)
-                 : "memory");
-}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 
 // Programmatic dependent launch.  A band pass lets the tile launch that
@@ -937,27 +933,36 @@ static __global__ void record_kernel(const StepParams P) { record_block(P, block
 // the row above, nz-nbc-2 first, which the tiles stored).  The tiles left the
 // stencil values of these rows (before the HABC) in the band scratch, so all
 // that runs here is the recurrence.  One warp per (strip of kStripW columns,
-// output field) marches down the rows: lane l holds column xs-2+l, so lanes
-// 2..29 are the strip, lanes 1 and 30 carry the recurrence of the
-// neighbouring columns, and lanes 0 and 31 supply values only.  Stencil and
-// step-start values arrive by cp.async, kMarchRows rows per chunk, one chunk
-// ahead.  A lane's column fixes its rule for every row: rim columns keep the
-// stencil value; the bottom edge reads the final value of row j-1 (z term);
-// corner cells add the x term of their neighbour towards the interior
-// (stencil value, phase A); the last bottom-left column (nbc) and
-// bottom-right chunk starts redo it with that neighbour's final value
-// (phase B).  Both rules are evaluated and selected, so a warp never
-// diverges.  Lane 1's values are wrong only when its column is a
-// bottom-right chunk start and lane 30's only when its column is nbc; no
-// strip lane reads either then.
-
+// output field) marches down the rows: lane l holds column xs - 4 + l (so that
+// rows arrive as 16-byte copies) and lanes 2..29 store.  Stencil and
+// step-start values arrive by cp.async, kMarchRows rows per chunk, kMarchBufs
+// chunks in flight.  Nothing a lane reads is written by the pass.  Every row is
+//   f = A + W (sx + ((-qz f' - qt_z ov) - qxt ov'))
+// with A = w pv; on the edge W = 1 - w and sx = -0 (which adds nothing), in a
+// corner W = (1 - w) / 2 and sx the x term.  Only f' and what follows from it
+// is on the chain (six operations a row); the rest is computed a group of rows
+// ahead.  A column that reads its neighbour's final value (the last
+// bottom-left column and the bottom-right chunk starts) has a chain of its own
+// beside the one every lane runs: it takes the neighbour's value of the row by
+// shuffle, which no other column waits for.  One B200, us per step against the first form (every rule
+// evaluated per row, the neighbour's value by shuffle on the chain): 2108 x 908
+// 39.9 -> 38.9, 3308 x 1508 74.6 -> 73.4; the pass alone takes about 12.6 us
+// at nbc 50, which is the corner strips' (edge strips finish in 4).
 
 constexpr int kMaxBandTab = 1024;                  // nbc + 2 <= this
-constexpr int kMarchStage = 2 * 2 * kMarchRows * 32;  // two chunks of (stencil, step-start) values
+constexpr int kMarchBufs = 3;
+constexpr int kMarchBuf = 2 * kMarchRows * 32;     // one chunk of stencil values, then of step-start values
+constexpr int kMarchStage = kMarchBufs * kMarchBuf;
 
 // Band-pass warps of one half step: strips x 3 (a velocity pass leaves the
 // third field's warps idle).
 __host__ __device__ constexpr int band_warp_count(int nx) { return band_block_count(nx) * 3; }
+
+// 16-byte asynchronous global -> shared copy; valid == false writes zeros.
+__device__ __forceinline__ void cp_async16(float* dst, const float* src, bool valid) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(valid ? 16 : 0)
+                 : "memory");
+}
 
 template <bool VEL>
 __device__ void band_march(const StepParams& P, const TiledArgs& T, int item, float* stage, float* stab) {
@@ -966,72 +971,117 @@ __device__ void band_march(const StepParams& P, const TiledArgs& T, int item, fl
     if (VEL && f == 2) return;  // block-uniform
     const int lane = threadIdx.x & 31;
     const int b = P.nbc, nx = P.nx, nz = P.nz, r0 = nx - b - 1, j0 = nz - b - 1;
-    const float* tab = P.w_tab[VEL ? f : 2];
-    for (int d = lane; d < b + 2; d += 32) stab[d] = __ldg(tab + d);
-    __syncwarp();
-    const int i = strip * kStripW - 2 + lane;
-    const bool col_ok = i >= 0 && i < nx;
+    const int xs = strip * kStripW, i = xs - 4 + lane;
     const int q = VEL ? VX + f : TXX + f;
     const int plane = VEL ? kBandVelPlane + f : f;
     const float* oin = in_field(P, q);
     float* oout = q == VX ? P.out[VX] : q == VZ ? P.out[VZ] : q == TXX ? P.out[TXX] : q == TZZ ? P.out[TZZ] : P.out[TXZ];
-    // the lane's rule
-    const bool rim = i <= 0 || i >= nx - 1;
-    const bool left = i >= 1 && i <= b;
-    const bool corner = left || (i >= r0 && i <= nx - 2);
-    const bool redo = i == b || (i > r0 - 1 && i <= nx - 2 && right_chunk_start(nx, b, i));
-    const int nb = min(max(lane + (left ? 1 : -1), 0), 31);  // neighbour towards the interior
-    const int dxi = max(min(i, nx - 1 - i), 0);
-    const size_t pitch = P.pitch;
-
+    const int n_chunks = (b + kMarchRows - 1) / kMarchRows;
+    // lane l copies columns 4 (l % 8) .. + 3 of rows l / 8, l / 8 + 4, ...
+    const int cc = xs - 4 + 4 * (lane & 7);
+    const bool c_ok = cc >= 0 && cc < nx;
     auto stage_chunk = [&](int c) {
-        float* buf = stage + (c & 1) * (2 * kMarchRows * 32);
-        for (int r = 0; r < kMarchRows; ++r) {
-            const int jb = c * kMarchRows + r;
-            const bool ok = col_ok && jb < b;
-            cp_async4(buf + r * 32 + lane, ok ? band_pre_at(P, T, plane, jb, i) : T.band_pre, ok);
-            cp_async4(buf + (kMarchRows + r) * 32 + lane, ok ? oin + cell(P, i, j0 + jb) : oin, ok);
+        if (c < n_chunks) {
+            float* buf = stage + (c % kMarchBufs) * kMarchBuf + 4 * (lane & 7);
+#pragma unroll
+            for (int r = lane >> 3, k = 0; k < kMarchRows / 4; r += 4, ++k) {
+                const int jb = c * kMarchRows + r;
+                const bool ok = c_ok && jb < b;
+                cp_async16(buf + r * 32, ok ? band_pre_at(P, T, plane, jb, cc) : T.band_pre, ok);
+                cp_async16(buf + (kMarchRows + r) * 32, ok ? oin + cell(P, cc, j0 + jb) : oin, ok);
+            }
         }
         cp_async_commit();
     };
-    float fprev = col_ok ? oout[cell(P, i, j0 - 1)] : 0.f;  // final and step-start values of the row above
-    float ovp = col_ok ? __ldg(oin + cell(P, i, j0 - 1)) : 0.f;
-    float* dst = oout + (col_ok ? cell(P, i, j0) : 0);
+#pragma unroll
+    for (int c = 0; c < kMarchBufs - 1; ++c) stage_chunk(c);
+    const float* tab = P.w_tab[VEL ? f : 2];
+    for (int d = lane; d < b + 2; d += 32) stab[d] = __ldg(tab + d);
+    const bool col_ok = i >= 0 && i < nx;
     const bool store = col_ok && lane >= 2 && lane < 2 + kStripW;
-    const int n_chunks = (b + kMarchRows - 1) / kMarchRows;
-    stage_chunk(0);
+    float fp = col_ok ? oout[cell(P, i, j0 - 1)] : 0.f;  // final and step-start values of the row above
+    float op = col_ok ? __ldg(oin + cell(P, i, j0 - 1)) : 0.f;
+    float* dst = oout + (col_ok ? cell(P, i, j0) : 0);
+    const size_t pitch = P.pitch;
+    const bool edge = xs - 2 > b && xs + kStripW - 3 < r0;  // every stored column is an edge column
+    // a corner strip: the lane's rule
+    const int r0i = i - r0;
+    const bool left = i >= 1 && i <= b, right = i >= r0 && i <= nx - 2, corner = left || right;
+    const bool rim = i <= 0 || i >= nx - 1;
+    const bool redo = (left && i == b) || (right && (r0i & (kChunk - 1)) == 0);
+    const bool any_redo = !edge && __any_sync(FULL, redo && store);
+    const float h = corner ? 0.5f : 1.f;
+    const int dx = max(min(min(i, nx - 1 - i), b + 1), 0);
+    // x neighbour towards the interior (lanes at the window's ends have none in it and store nothing)
+    const int l1 = min(max(lane + (left ? 1 : right ? -1 : 0), 0), 31);
+    float fr = fp;  // the chain of the columns that read a final value
     for (int c = 0; c < n_chunks; ++c) {
-        if (c + 1 < n_chunks) {
-            stage_chunk(c + 1);
-            cp_async_wait<1>();
-        } else {
-            cp_async_wait<0>();
+        cp_async_wait<kMarchBufs - 2>();
+        __syncwarp();  // the chunk is here for every lane, and the one before it is done with
+        stage_chunk(c + kMarchBufs - 1);
+        const float* pvs = stage + (c % kMarchBufs) * kMarchBuf;
+        const float* ovs = pvs + kMarchRows * 32;
+        const int rows = min(kMarchRows, b - c * kMarchRows), d0 = b - c * kMarchRows;  // d0: distance to the bottom
+        constexpr int G = 8;
+        if (edge) {
+#pragma unroll
+            for (int g = 0; g < kMarchRows; g += G) {
+                if (g >= rows) break;
+                float A[G], W[G], t1[G], t2[G];
+#pragma unroll
+                for (int r = 0; r < G; ++r) {  // rows past the band read zeros
+                    const float w = stab[max(d0 - g - r, 0)], ov = ovs[(g + r) * 32 + lane];
+                    A[r] = fmul(w, pvs[(g + r) * 32 + lane]);
+                    W[r] = fsub(1.f, w);
+                    t1[r] = fmul(P.qt_z, ov);
+                    t2[r] = fmul(P.qxt, op);
+                    op = ov;
+                }
+#pragma unroll
+                for (int r = 0; r < G; ++r)
+                    if (g + r < rows) {
+                        fp = fadd(A[r], fmul(W[r], fsub(fsub(fmul(-P.qz, fp), t1[r]), t2[r])));
+                        if (store) *dst = fp;
+                        dst += pitch;
+                    }
+            }
+            continue;
         }
-        __syncwarp();
-        const float* buf = stage + (c & 1) * (2 * kMarchRows * 32);
-        const int rows = min(kMarchRows, b - c * kMarchRows);
-#pragma unroll 4
-        for (int r = 0; r < rows; ++r) {
-            const int j = j0 + c * kMarchRows + r;
-            const float pv = buf[r * 32 + lane];
-            const float ov = buf[(kMarchRows + r) * 32 + lane];
-            const float w = stab[min(min(dxi, nz - 1 - j), b + 1)];
-            const float pv_nb = __shfl_sync(FULL, pv, nb);
-            const float ov_nb = __shfl_sync(FULL, ov, nb);
-            const float sz = edge_sum(P.qz, P.qt_z, P.qxt, fprev, ov, ovp);
-            const float fc = blend_corner(w, pv, edge_sum(P.qx, P.qt_x, P.qxt, pv_nb, ov, ov_nb), sz);
-            const float fe = blend_edge(w, pv, sz);
-            const float fa = rim ? pv : (corner ? fc : fe);
-            const float fa_nb = __shfl_sync(FULL, fa, nb);
-            const float fb = blend_corner(w, pv, edge_sum(P.qx, P.qt_x, P.qxt, fa_nb, ov, ov_nb), sz);
-            const float fin = redo ? fb : fa;
-            if (store) *dst = fin;
-            dst += pitch;
-            fprev = fin;
-            ovp = ov;
+#pragma unroll 1
+        for (int g = 0; g < rows; g += G) {
+            float A[G], W[G], t1[G], t2[G], sx[G], u1[G], u2[G];
+#pragma unroll
+            for (int r = 0; r < G; ++r) {
+                const int k = (g + r) * 32;
+                const float pv = pvs[k + lane], ov = ovs[k + lane], ovn = ovs[k + l1];
+                const float w = stab[min(dx, max(d0 - g - r, 0))];
+                u1[r] = fmul(P.qt_x, ov);
+                u2[r] = fmul(P.qxt, ovn);
+                const float s = fsub(fsub(fmul(-P.qx, pvs[k + l1]), u1[r]), u2[r]);
+                sx[r] = corner ? s : -0.f;
+                A[r] = rim ? pv : fmul(w, pv);
+                W[r] = fmul(fsub(1.f, w), h);
+                t1[r] = fmul(P.qt_z, ov);
+                t2[r] = fmul(P.qxt, op);
+                op = ov;
+            }
+#pragma unroll
+            for (int r = 0; r < G; ++r)
+                if (g + r < rows) {
+                    const float v = fadd(A[r], fmul(W[r], fadd(sx[r], fsub(fsub(fmul(-P.qz, fp), t1[r]), t2[r]))));
+                    fp = rim ? A[r] : v;
+                    float out = fp;
+                    if (any_redo) {
+                        const float x = fsub(fsub(fmul(-P.qx, __shfl_sync(FULL, fp, l1)), u1[r]), u2[r]);
+                        fr = fadd(A[r], fmul(W[r], fadd(x, fsub(fsub(fmul(-P.qz, fr), t1[r]), t2[r]))));
+                        out = redo ? fr : fp;
+                    }
+                    if (store) *dst = out;
+                    dst += pitch;
+                }
         }
-        __syncwarp();  // every lane is done with this chunk's buffer
     }
+    cp_async_wait<0>();
 }
 
 // The band pass of one half step: one warp per (strip, field) (P, T as for
