@@ -815,8 +815,11 @@ int run_steps_split(Shot& s, Medium& m, Wavefield& w, int n_steps, Profile* prof
     auto& C = ctx();
     const bool iso = s.dtx == s.dtz;
     const Launch L = launch_shape<M>(m.nx, m.nz, s.nbc, iso, m.fs != 0);
-    if (int rc = raise_smem_limit(fomo::velocity_kernel<M>, L.smem_v)) return rc;
-    if (int rc = raise_smem_limit(fomo::stress_kernel<M>, L.smem_s)) return rc;
+    const bool gen = fomo::tiles_generic(m.fs != 0, s.nbc);
+    auto* const velocity = gen ? fomo::velocity_kernel<M, true> : fomo::velocity_kernel<M, false>;
+    auto* const stress = gen ? fomo::stress_kernel<M, true> : fomo::stress_kernel<M, false>;
+    if (int rc = raise_smem_limit(velocity, L.smem_v)) return rc;
+    if (int rc = raise_smem_limit(stress, L.smem_s)) return rc;
     if (w.map_M != M)
         if (int rc = make_maps<M>(w)) return rc;
     if (int rc = ensure_buoyancy(m, s.dtx, s.dtz)) return rc;
@@ -830,6 +833,7 @@ int run_steps_split(Shot& s, Medium& m, Wavefield& w, int n_steps, Profile* prof
     T.tiles_x = L.tiles_x;
     T.x_last = L.x_last;
     T.prefetch_ahead = fomo::prefetch_distance(sm_count());
+    T.first_wave = fomo::first_wave_blocks(sm_count());
     const int rec_blocks = (s.n_rec + fomo::kThreads - 1) / fomo::kThreads;
     CUDA_TRY(cudaEventRecord(C.ev0, C.stream));
     const int k_begin = s.k_done + 1, k_end = std::min(s.nt, s.k_done + n_steps);
@@ -857,7 +861,7 @@ int run_steps_split(Shot& s, Medium& m, Wavefield& w, int n_steps, Profile* prof
         vm.b2 = m.buoy_maps[2];
         vm.b3 = m.buoy_maps[3];
         // profiled launches stay serialised (events sit between them)
-        CUDA_TRY(launch_tiles(fomo::velocity_kernel<M>, vblocks, L.smem_v, C.stream, !prof && k > k_begin, P, T, vm));
+        CUDA_TRY(launch_tiles(velocity, vblocks, L.smem_v, C.stream, !prof && k > k_begin, P, T, vm));
         if (prof && prof->end(C.stream)) return fail(FOMO_ECUDA, "profiling event failed");
         if (prof && prof->add(C.stream, 2)) return fail(FOMO_ECUDA, "profiling event failed");
         fomo::band_kernel<true><<<L.n_band, 32, 0, C.stream>>>(P, T);
@@ -878,7 +882,7 @@ int run_steps_split(Shot& s, Medium& m, Wavefield& w, int n_steps, Profile* prof
         sm.lam = m.mod_maps[0];
         sm.mu = m.mod_maps[1];
         sm.mxz = m.mod_maps[2];
-        CUDA_TRY(launch_tiles(fomo::stress_kernel<M>, L.n_tile, L.smem_s, C.stream, !prof, P, T, sm));
+        CUDA_TRY(launch_tiles(stress, L.n_tile, L.smem_s, C.stream, !prof, P, T, sm));
         if (prof && prof->end(C.stream)) return fail(FOMO_ECUDA, "profiling event failed");
         if (prof && prof->add(C.stream, 3)) return fail(FOMO_ECUDA, "profiling event failed");
         fomo::band_kernel<false><<<L.n_band, 32, 0, C.stream>>>(P, T);
@@ -1553,12 +1557,16 @@ int noalloc_loop(const fomo::StepParams& P0, fomo::TiledArgs T, float* fields, i
     for (int q = 0; q < 4; ++q)
         if (int rc = encode_map(&bm[q], buoy[q], nx, nz, pitch, fomo::kTX, fomo::kTZ)) return rc;
     const Launch L = launch_shape<M>(nx, nz, P0.nbc, iso, P0.fs != 0);
-    if (int rc = raise_smem_limit(fomo::velocity_kernel<M>, L.smem_v)) return rc;
-    if (int rc = raise_smem_limit(fomo::stress_kernel<M>, L.smem_s)) return rc;
+    const bool gen = fomo::tiles_generic(P0.fs != 0, P0.nbc);
+    auto* const velocity = gen ? fomo::velocity_kernel<M, true> : fomo::velocity_kernel<M, false>;
+    auto* const stress = gen ? fomo::stress_kernel<M, true> : fomo::stress_kernel<M, false>;
+    if (int rc = raise_smem_limit(velocity, L.smem_v)) return rc;
+    if (int rc = raise_smem_limit(stress, L.smem_s)) return rc;
     T.n_tile_blocks = L.n_tile;
     T.tiles_x = L.tiles_x;
     T.x_last = L.x_last;
     T.prefetch_ahead = fomo::prefetch_distance(sm_count());
+    T.first_wave = fomo::first_wave_blocks(sm_count());
     const int rec_blocks = (n_rec + fomo::kThreads - 1) / fomo::kThreads;
     int cur = 0;
     for (int k = 1; k <= nt; ++k) {
@@ -1579,7 +1587,7 @@ int noalloc_loop(const fomo::StepParams& P0, fomo::TiledArgs T, float* fields, i
         vm.b1 = bm[1];
         vm.b2 = bm[2];
         vm.b3 = bm[3];
-        fomo::velocity_kernel<M><<<L.n_tile + (P.rec_k ? rec_blocks : 0), fomo::kThreads, L.smem_v, st>>>(P, T, vm);
+        velocity<<<L.n_tile + (P.rec_k ? rec_blocks : 0), fomo::kThreads, L.smem_v, st>>>(P, T, vm);
         fomo::band_kernel<true><<<L.n_band, 32, 0, st>>>(P, T);
         P.in[fomo::VX] = field(b, fomo::VX);
         P.in[fomo::VZ] = field(b, fomo::VZ);
@@ -1595,7 +1603,7 @@ int noalloc_loop(const fomo::StepParams& P0, fomo::TiledArgs T, float* fields, i
         sm.lam = mod[0];
         sm.mu = mod[1];
         sm.mxz = mod[2];
-        fomo::stress_kernel<M><<<L.n_tile, fomo::kThreads, L.smem_s, st>>>(P, T, sm);
+        stress<<<L.n_tile, fomo::kThreads, L.smem_s, st>>>(P, T, sm);
         fomo::band_kernel<false><<<L.n_band, 32, 0, st>>>(P, T);
         cur = b;
     }

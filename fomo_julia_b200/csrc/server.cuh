@@ -187,19 +187,21 @@ size_t batch_smem_any(int M, bool vel, int nbc, bool iso, bool fs) {
 }
 
 template <int M>
-int set_batch_smem_M(size_t v, size_t s) {
-    if (int rc = raise_smem_limit(fomo::batch_velocity_kernel<M>, v)) return rc;
-    return raise_smem_limit(fomo::batch_stress_kernel<M>, s);
+int set_batch_smem_M(size_t v, size_t s, bool gen) {
+    if (int rc = gen ? raise_smem_limit(fomo::batch_velocity_kernel<M, true>, v)
+                     : raise_smem_limit(fomo::batch_velocity_kernel<M, false>, v))
+        return rc;
+    return gen ? raise_smem_limit(fomo::batch_stress_kernel<M, true>, s) : raise_smem_limit(fomo::batch_stress_kernel<M, false>, s);
 }
 
-int set_batch_smem(int M, size_t v, size_t s) {
+int set_batch_smem(int M, size_t v, size_t s, bool gen) {
     switch (M) {
-        case 1: return set_batch_smem_M<1>(v, s);
-        case 2: return set_batch_smem_M<2>(v, s);
-        case 3: return set_batch_smem_M<3>(v, s);
-        case 4: return set_batch_smem_M<4>(v, s);
-        case 5: return set_batch_smem_M<5>(v, s);
-        case 6: return set_batch_smem_M<6>(v, s);
+        case 1: return set_batch_smem_M<1>(v, s, gen);
+        case 2: return set_batch_smem_M<2>(v, s, gen);
+        case 3: return set_batch_smem_M<3>(v, s, gen);
+        case 4: return set_batch_smem_M<4>(v, s, gen);
+        case 5: return set_batch_smem_M<5>(v, s, gen);
+        case 6: return set_batch_smem_M<6>(v, s, gen);
     }
     return fail(FOMO_EINVAL, "M=%d not supported", M);
 }
@@ -212,6 +214,7 @@ struct LaunchSet {
     std::shared_ptr<fomo::BatchStrLaunch> ls;  // and of the stress launches
     int grid_v = 0, grid_s = 0, grid_b = 0;    // velocity tiles + receivers, stress tiles, band passes
     size_t smem_v = 0, smem_s = 0;
+    bool gen = false;                          // some shot has generic tiles
 };
 
 // Shots of one FD order in flight that run the fused step: one launch per
@@ -298,8 +301,12 @@ bool march_ok(const Request& r) {
 // beside the band pass just before it, see launch_tiles).
 template <int M>
 void launch_batch_M(bool vel, const LaunchSet& S, cudaStream_t st, bool after_band) {
-    if (vel) launch_tiles(fomo::batch_velocity_kernel<M>, S.grid_v, S.smem_v, st, after_band, *S.lv);
-    else launch_tiles(fomo::batch_stress_kernel<M>, S.grid_s, S.smem_s, st, after_band, *S.ls);
+    if (vel)
+        launch_tiles(S.gen ? fomo::batch_velocity_kernel<M, true> : fomo::batch_velocity_kernel<M, false>, S.grid_v, S.smem_v, st,
+                     after_band, *S.lv);
+    else
+        launch_tiles(S.gen ? fomo::batch_stress_kernel<M, true> : fomo::batch_stress_kernel<M, false>, S.grid_s, S.smem_s, st,
+                     after_band, *S.ls);
 }
 
 void launch_batch(bool vel, const LaunchSet& S, cudaStream_t st, bool after_band) {
@@ -821,6 +828,7 @@ class Server {
                 const Launch L = shape_of(r);
                 S.smem_v = std::max(S.smem_v, L.smem_v);
                 S.smem_s = std::max(S.smem_s, L.smem_s);
+                S.gen = S.gen || fomo::tiles_generic(r.med->fs != 0, r.nbc);
                 S.lv->shot[t] = r.vel;
                 S.ls->shot[t] = r.str;
                 for (int c = 0; c < 2; ++c) {
@@ -838,6 +846,7 @@ class Server {
             H.n_shots = (int)(j - i);
             H.n_groups = n_groups;
             H.pf_ahead = fomo::prefetch_distance(sm_count());
+            H.first_wave = fomo::first_wave_blocks(sm_count());
             H.total_band = band;
             H.total_tile = tile;
             S.ls->H = H;
@@ -846,7 +855,7 @@ class Server {
             S.grid_v = tile + rec;
             S.grid_s = tile;
             S.grid_b = band;
-            if (int rc = set_batch_smem(S.M, S.smem_v, S.smem_s)) return rc;
+            if (int rc = set_batch_smem(S.M, S.smem_v, S.smem_s, S.gen)) return rc;
             sets_.push_back(S);
             i = j;
         }

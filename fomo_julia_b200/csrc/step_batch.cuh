@@ -64,6 +64,7 @@ struct BatchHead {
     int* advance;                     // the other half step's counter of the set (block 0 advances it)
     int kpar;                         // parity of that batch step (the host knows it when it launches)
     int pf_ahead;                     // tile blocks between a block and the one whose boxes it prefetches
+    int first_wave;                   // blocks resident at once (nothing prefetches for them)
     int n_shots, n_groups;
     int total_band, total_tile;
     int rec_off[kShotsPerLaunch + 1]; // first receiver block of each shot
@@ -212,7 +213,7 @@ struct BatchPrefetch {
     }
 };
 
-template <int M>
+template <int M, bool GEN>
 __global__ void __launch_bounds__(kThreads, kTileBlocks<M>) batch_velocity_kernel(const __grid_constant__ BatchVelLaunch L) {
     extern __shared__ __align__(128) float smem[];
     block0_advance(L.H);
@@ -233,20 +234,22 @@ __global__ void __launch_bounds__(kThreads, kTileBlocks<M>) batch_velocity_kerne
     const StepParams& P = S.P[c];
     const TileKind k = classify(P, S.T, it.local);
     if (reads_band_rows(P, k.z0)) grid_dep_wait();
-    if (k.generic) {
+    if (GEN && k.generic) {
         if (!live) return;
         edge_tile<M, true>(P, S.T, k.x0, k.z0, k.x_end, smem, wavelet_at(S, ks));
     } else {
         const int s = it.shot;
         const VelMapRefs mp{&L.tau[s][c][0], &L.tau[s][c][1], &L.tau[s][c][2], &L.v[s][c][0], &L.v[s][c][1],
                             &L.b[s][0],      &L.b[s][1],      &L.b[s][2],      &L.b[s][3]};
-        const BatchPrefetch<M, true, BatchVelLaunch> pf{L, L.H.pf_ahead > 0 ? (int)blockIdx.x + L.H.pf_ahead : 1 << 30};
+        const BatchPrefetch<M, true, BatchVelLaunch> pf{L, L.H.pf_ahead > 0 && (int)blockIdx.x + L.H.pf_ahead >= L.H.first_wave
+                                                                       ? (int)blockIdx.x + L.H.pf_ahead
+                                                                       : 1 << 30};
         fast_vel<M>(P, S.T, mp, k.x0, k.z0, k.x_end, k.band, k.rim, smem, wavelet_at(S, ks), -1, live, pf);
     }
     if (threadIdx.x == 0 && live && ((ks - 1) & 1) != c) atomicCAS(S.T.status, 0, kErrBatchParity);
 }
 
-template <int M>
+template <int M, bool GEN>
 __global__ void __launch_bounds__(kThreads, kTileBlocks<M>) batch_stress_kernel(const __grid_constant__ BatchStrLaunch L) {
     extern __shared__ __align__(128) float smem[];
     block0_advance(L.H);
@@ -259,14 +262,16 @@ __global__ void __launch_bounds__(kThreads, kTileBlocks<M>) batch_stress_kernel(
     const StepParams& P = S.P[a];
     const TileKind k = classify(P, S.T, it.local);
     if (reads_band_rows(P, k.z0)) grid_dep_wait();
-    if (k.generic) {
+    if (GEN && k.generic) {
         if (!live) return;
         edge_tile<M, false>(P, S.T, k.x0, k.z0, k.x_end, smem, wavelet_at(S, ks));
     } else {
         const int s = it.shot;
         const StrMapRefs mp{&L.v[s][b][0],   &L.v[s][b][1],   &L.tau[s][a][0], &L.tau[s][a][1],
                             &L.tau[s][a][2], &L.mod[s][0],    &L.mod[s][1],    &L.mod[s][2]};
-        const BatchPrefetch<M, false, BatchStrLaunch> pf{L, L.H.pf_ahead > 0 ? (int)blockIdx.x + L.H.pf_ahead : 1 << 30};
+        const BatchPrefetch<M, false, BatchStrLaunch> pf{L, L.H.pf_ahead > 0 && (int)blockIdx.x + L.H.pf_ahead >= L.H.first_wave
+                                                                       ? (int)blockIdx.x + L.H.pf_ahead
+                                                                       : 1 << 30};
         fast_str<M>(P, S.T, mp, k.x0, k.z0, k.x_end, k.band, k.rim, smem, wavelet_at(S, ks), -1, live, pf);
     }
     if (threadIdx.x == 0 && live && ((ks - 1) & 1) != a) atomicCAS(S.T.status, 0, kErrBatchParity);

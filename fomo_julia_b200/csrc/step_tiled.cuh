@@ -71,6 +71,7 @@ struct TiledArgs {
     int n_tile_blocks, tiles_x;
     int x_last;          // first column of the last tile of a row (a multiple of 4)
     int prefetch_ahead;  // tile blocks between a fast tile and the tile it prefetches (0 = none)
+    int first_wave;      // blocks resident at once: earlier ones load their own boxes right away
 };
 
 __device__ __forceinline__ int tile_x0(const TiledArgs& T, int tx) {
@@ -525,6 +526,32 @@ __device__ __forceinline__ float4 side_weights(const StepParams& P, const float*
     return make_float4(w[0], w[1], w[2], w[3]);
 }
 
+// side_rules as a call, for the tile kernels: six inlined copies a kernel were
+// a third of its code, and a launch starts with a cold instruction cache.  The
+// rules' parameters come by value, since a call cannot read the kernel's.
+struct SideParams {
+    int nx, nz, nbc, fs;
+    float qx, qt_x, qxt, neg_zero;
+};
+__device__ __forceinline__ SideParams side_params(const StepParams& P) {
+    return {P.nx, P.nz, P.nbc, P.fs, P.qx, P.qt_x, P.qxt, P.neg_zero};
+}
+static __device__ __noinline__ float4 side_rules_call(SideParams S, const float* tab, int x, int j, bool left, bool right, float4 n,
+                                                      float4 o) {
+    StepParams P;
+    P.nx = S.nx;
+    P.nz = S.nz;
+    P.nbc = S.nbc;
+    P.fs = S.fs;
+    P.qx = S.qx;
+    P.qt_x = S.qt_x;
+    P.qxt = S.qxt;
+    P.neg_zero = S.neg_zero;
+    side_rules(P, left, right, side_weights(P, tab, x, j), x, j, n, o);
+    return n;
+}
+
+
 // L2 prefetch of the boxes of tile `tile` when it is a fast tile of this
 // launch (defined after classify).  The single-shot fast tiles pass
 // pf_tile = their block + T.prefetch_ahead, so that tile's DRAM reads start
@@ -650,8 +677,8 @@ __device__ __forceinline__ void fast_vel(const StepParams& P, const TiledArgs& T
 #pragma unroll
         for (int rr = 0; rr < 2; ++rr) {
             const int po = (2 * rp + rr) * kTX + xr, j = zt + rr;
-            side_rules(P, left, right, side_weights(P, P.w_tab[0], x, j), x, j, ox[rr], lds4(p_vx + po));
-            side_rules(P, left, right, side_weights(P, P.w_tab[1], x, j), x, j, oz[rr], lds4(p_vz + po));
+            ox[rr] = side_rules_call(side_params(P), P.w_tab[0], x, j, left, right, ox[rr], lds4(p_vx + po));
+            oz[rr] = side_rules_call(side_params(P), P.w_tab[1], x, j, left, right, oz[rr], lds4(p_vz + po));
         }
     }
     if (x < x_end) {
@@ -771,10 +798,9 @@ __device__ __forceinline__ void fast_str(const StepParams& P, const TiledArgs& T
 #pragma unroll
         for (int rr = 0; rr < 2; ++rr) {
             const int po = (2 * rp + rr) * kTX + xr, j = zt + rr;
-            const float4 w = side_weights(P, P.w_tab[2], x, j);
-            side_rules(P, left, right, w, x, j, oxx[rr], lds4(p_xx + po));
-            side_rules(P, left, right, w, x, j, ozz[rr], lds4(p_zz + po));
-            side_rules(P, left, right, w, x, j, oxz[rr], lds4(p_xz + po));
+            oxx[rr] = side_rules_call(side_params(P), P.w_tab[2], x, j, left, right, oxx[rr], lds4(p_xx + po));
+            ozz[rr] = side_rules_call(side_params(P), P.w_tab[2], x, j, left, right, ozz[rr], lds4(p_zz + po));
+            oxz[rr] = side_rules_call(side_params(P), P.w_tab[2], x, j, left, right, oxz[rr], lds4(p_xz + po));
         }
     }
     if (x < x_end) {
@@ -829,7 +855,11 @@ __device__ __forceinline__ bool reads_band_rows(const StepParams& P, int z0) {
 // 4552 x 3927 grid on 148 SMs, the velocity launch was fastest 260-370 blocks
 // ahead (113.8 us at one wave, 740; 140.9 us at 1480) and the stress launch
 // 185-370 ahead (148.8 us at 92, 150 us at 740).
+// Blocks of the first wave (first_wave) start their own copies at once, so
+// nothing prefetches for them: 2108 x 908 35.1 -> 34.8 us per step, 4552 x 3927
+// 212.2 -> 211.8.
 __host__ inline int prefetch_distance(int sm_count) { return 2 * sm_count; }
+__host__ inline int first_wave_blocks(int sm_count) { return kTileBlocks<1> * sm_count; }
 
 template <int M>
 __device__ void prefetch_vel(const StepParams& P, const TiledArgs& T, const VelMapRefs& mp, int tile) {
@@ -880,7 +910,14 @@ __device__ inline void record_block(const StepParams& P, int rblock, int rec_k) 
 }
 
 // ---------------------------------------------------------------- kernels
-template <int M>
+// GEN: the launch has generic tiles (no free surface, or HABC bands wider than
+// a tile allows: tiles_generic).  Launches without them run kernels without
+// that path's code, half of the whole.  Measured with side_rules_call, us per
+// step on one B200: 2108 x 908 38.9 -> 35.1, 3308 x 1508 73.4 -> 68.7,
+// 4552 x 3927 217.0 -> 213.0.
+__host__ __device__ constexpr bool tiles_generic(bool fs, int nbc) { return !fs || nbc + 6 > kTX; }
+
+template <int M, bool GEN>
 __global__ void __launch_bounds__(kThreads, kTileBlocks<M>) velocity_kernel(const __grid_constant__ StepParams P, const __grid_constant__ TiledArgs T,
                                                             const __grid_constant__ VelMaps maps) {
     extern __shared__ __align__(128) float smem[];
@@ -888,9 +925,9 @@ __global__ void __launch_bounds__(kThreads, kTileBlocks<M>) velocity_kernel(cons
     if (bid < T.n_tile_blocks) {
         const TileKind k = classify(P, T, bid);
         if (reads_band_rows(P, k.z0)) grid_dep_wait();
-        if (k.generic) edge_tile<M, true>(P, T, k.x0, k.z0, k.x_end, smem, P.src_w);
+        if (GEN && k.generic) edge_tile<M, true>(P, T, k.x0, k.z0, k.x_end, smem, P.src_w);
         else fast_vel<M>(P, T, refs_of(maps), k.x0, k.z0, k.x_end, k.band, k.rim, smem, P.src_w,
-                         T.prefetch_ahead > 0 ? bid + T.prefetch_ahead : -1);
+                         T.prefetch_ahead > 0 && bid + T.prefetch_ahead >= T.first_wave ? bid + T.prefetch_ahead : -1);
         return;
     }
     grid_dep_wait();  // receivers may sit in the band rows
@@ -910,7 +947,7 @@ __device__ __forceinline__ int stress_tile(const StepParams& P, const TiledArgs&
     return b < n_early ? n_early - 1 - b : b;
 }
 
-template <int M>
+template <int M, bool GEN>
 __global__ void __launch_bounds__(kThreads, kTileBlocks<M>) stress_kernel(const __grid_constant__ StepParams P, const __grid_constant__ TiledArgs T,
                                                           const __grid_constant__ StrMaps maps) {
     extern __shared__ __align__(128) float smem[];
@@ -918,9 +955,9 @@ __global__ void __launch_bounds__(kThreads, kTileBlocks<M>) stress_kernel(const 
     if (bid < T.n_tile_blocks) {
         const TileKind k = classify(P, T, stress_tile(P, T, bid));
         if (reads_band_rows(P, k.z0)) grid_dep_wait();
-        if (k.generic) edge_tile<M, false>(P, T, k.x0, k.z0, k.x_end, smem, P.src_w);
+        if (GEN && k.generic) edge_tile<M, false>(P, T, k.x0, k.z0, k.x_end, smem, P.src_w);
         else fast_str<M>(P, T, refs_of(maps), k.x0, k.z0, k.x_end, k.band, k.rim, smem, P.src_w,
-                         T.prefetch_ahead > 0 ? stress_tile(P, T, bid + T.prefetch_ahead) : -1);
+                         T.prefetch_ahead > 0 && bid + T.prefetch_ahead >= T.first_wave ? stress_tile(P, T, bid + T.prefetch_ahead) : -1);
     }
 }
 
@@ -1184,8 +1221,7 @@ __host__ size_t tiled_smem_bytes(bool vel, int nbc, bool iso, bool fs) {
     const int npoint = vel ? (iso ? 4 : 6) : 6;
     const size_t interior = ((size_t)nin * G::BOXS + (size_t)npoint * kPBox) * 4 + 16;
     const size_t edge = ((size_t)nin * (G::RW + 2 * M) * (G::RH + 2 * M) + (size_t)nout * G::RW * G::RH) * 4;
-    const bool generic = !fs || nbc + 6 > kTX;
-    return generic ? std::max(interior, edge) : interior;
+    return tiles_generic(fs, nbc) ? std::max(interior, edge) : interior;
 }
 
 }  // namespace fomo
