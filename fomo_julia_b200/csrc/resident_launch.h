@@ -56,16 +56,17 @@ __host__ __device__ constexpr int resident_mail_items(int M, int h_max) { return
 // band's scratch (step-start values of its b rows and the row above; x terms of
 // the corners), the top
 // band's (no free surface: values before the band rule of rows 0..b+1, one
-// row of step-start values; results), the weight tables, the receiver list
-// and a few words.
+// row of step-start values; results), the medium where it fits, the receiver
+// list, the exchange's table, the weight tables and a few words.
 __host__ __device__ constexpr size_t resident_plane(int M, int h) { return (size_t)(h + 2 * M + 1) * resident_pitch(M); }
 __host__ __device__ constexpr size_t resident_bottom_floats(int b) { return (size_t)3 * (2 * b + 1) * kRW; }
 __host__ __device__ constexpr size_t resident_top_floats(int b) { return (size_t)3 * (2 * b + 3) * kRW; }
 __host__ __device__ constexpr size_t resident_tail_floats(int b) { return (size_t)3 * kRW + 3 * (b + 2) + 2 * kRRecCap + 16; }
+__host__ __device__ constexpr size_t resident_table_floats(int M, int h) { return 2 * (size_t)(2 * M * h + 2 * M * kRW); }
 __host__ __device__ constexpr size_t resident_med_floats(int h, bool iso) { return (size_t)(iso ? 5 : 7) * h * kRW; }
 __host__ __device__ constexpr size_t resident_smem_floats(int M, int b, int h, bool bottom, bool top, bool med, bool iso) {
     return 5 * resident_plane(M, h) + (bottom ? resident_bottom_floats(b) : 0) + (top ? resident_top_floats(b) : 0) +
-           (med ? resident_med_floats(h, iso) : 0) + resident_tail_floats(b);
+           (med ? resident_med_floats(h, iso) : 0) + resident_table_floats(M, h) + resident_tail_floats(b);
 }
 
 // Item `idx` of the messages a region of h rows and w columns exchanges
@@ -122,6 +123,7 @@ inline ResidentPlan resident_plan(int nx, int nz, int M, int nbc, bool fs, bool 
     // first and last wide enough for the side band and the columns it reads.
     const int G = (nx + 3) / 4, per = kRW / 4, S = (G + per - 1) / per;
     if (S > slots || S >= kRMaxEdges) return p;
+    if (nx - 2 * nbc - 1 < 4) return p;  // a thread's four columns hold one band's at most
     std::vector<int> g(S);
     for (int s = 0; s < S; ++s) g[s] = (int)((long)G * (s + 1) / S - (long)G * s / S);
     if (S > 1) {

@@ -465,54 +465,81 @@ __device__ __forceinline__ void zderiv(const StepParams& P, const float4 (&wz)[2
 // them.  Registers and shuffles instead: us per step, one B200, 4552 x 3927
 // 255.8 -> 217.8 (80 B a cell at the measured copy bandwidth), 3308 x 1508
 // 107.6 -> 74.6, 2108 x 908 71.4 -> 39.9, 508 x 308 52.4 -> 28.7.
-__device__ __forceinline__ void side_rules(const StepParams& P, bool left, bool right, const float4& w, int x, int j, float4& n,
-                                           const float4& o) {
+//
+// NF fields at once (the same row and columns), so that their shuffles and
+// chains overlap.  LEFT: the left band, reading i+1; else the right band.
+template <int NF, bool LEFT>
+__device__ __forceinline__ void side_band(const StepParams& P, const float4 (&w)[NF], int x, int j, const float4 (&pre)[NF],
+                                          const float4 (&o)[NF], float4 (&n)[NF]) {
     constexpr unsigned FULL = 0xffffffffu;
     const int b = P.nbc, r0 = P.nx - b - 1;
     const bool row = j >= (P.fs ? b : 1) && j <= P.nz - b - 2;
-    const float4 pre = n;
     const float2 nq = make_float2(-P.qx, -P.qx), qt = make_float2(P.qt_x, P.qt_x), qxt = make_float2(P.qxt, P.qxt);
     const float2 one = make_float2(1.f, 1.f);
-    const float2 Al = mul2(P, lo2(w), lo2(pre)), Ah = mul2(P, hi2(w), hi2(pre));
-    const float2 Wl = sub2(one, lo2(w)), Wh = sub2(one, hi2(w));
-    const float2 tl = mul2(P, qt, lo2(o)), th = mul2(P, qt, hi2(o));
-    if (left) {
-        const float nr = __shfl_down_sync(FULL, pre.x, 1, 16), orr = __shfl_down_sync(FULL, o.x, 1, 16);
-        const float2 sl = sub2(sub2(mul2(P, nq, make_float2(pre.y, pre.z)), tl), mul2(P, qxt, make_float2(o.y, o.z)));
-        const float2 sh = sub2(sub2(mul2(P, nq, make_float2(pre.w, nr)), th), mul2(P, qxt, make_float2(o.w, orr)));
-        const float2 fl = add2(Al, mul2(P, Wl, sl)), fh = add2(Ah, mul2(P, Wh, sh));
-        if (row && x >= 1 && x <= b) n.x = fl.x;
-        if (row && x + 1 <= b) n.y = fl.y;
-        if (row && x + 2 <= b) n.z = fh.x;
-        if (row && x + 3 <= b) n.w = fh.y;
+    bool m[4];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) m[c] = row && (LEFT ? x + c >= 1 && x + c <= b : x + c >= r0 && x + c <= P.nx - 2);
+    float ne[NF], oe[NF];  // the neighbouring thread's column
+#pragma unroll
+    for (int f = 0; f < NF; ++f) {
+        ne[f] = LEFT ? __shfl_down_sync(FULL, pre[f].x, 1, 16) : __shfl_up_sync(FULL, pre[f].w, 1, 16);
+        oe[f] = LEFT ? __shfl_down_sync(FULL, o[f].x, 1, 16) : __shfl_up_sync(FULL, o[f].w, 1, 16);
     }
-    if (right) {
-        const float nl = __shfl_up_sync(FULL, pre.w, 1, 16), ol = __shfl_up_sync(FULL, o.w, 1, 16);
-        const float2 ql = mul2(P, qxt, make_float2(ol, o.x)), qh = mul2(P, qxt, make_float2(o.y, o.z));
-        const float2 sl = sub2(sub2(mul2(P, nq, make_float2(nl, pre.x)), tl), ql);
-        const float2 sh = sub2(sub2(mul2(P, nq, make_float2(pre.y, pre.z)), th), qh);
-        float2 fl = add2(Al, mul2(P, Wl, sl)), fh = add2(Ah, mul2(P, Wh, sh));
+    float2 fl[NF], fh[NF], Al[NF], Ah[NF], Wl[NF], Wh[NF], tl[NF], th[NF], ql[NF], qh[NF];
+#pragma unroll
+    for (int f = 0; f < NF; ++f) {
+        const float2 nl = LEFT ? make_float2(pre[f].y, pre[f].z) : make_float2(ne[f], pre[f].x);
+        const float2 nh = LEFT ? make_float2(pre[f].w, ne[f]) : make_float2(pre[f].y, pre[f].z);
+        const float2 ol = LEFT ? make_float2(o[f].y, o[f].z) : make_float2(oe[f], o[f].x);
+        const float2 oh = LEFT ? make_float2(o[f].w, oe[f]) : make_float2(o[f].y, o[f].z);
+        Al[f] = mul2(P, lo2(w[f]), lo2(pre[f]));
+        Ah[f] = mul2(P, hi2(w[f]), hi2(pre[f]));
+        Wl[f] = sub2(one, lo2(w[f]));
+        Wh[f] = sub2(one, hi2(w[f]));
+        tl[f] = mul2(P, qt, lo2(o[f]));
+        th[f] = mul2(P, qt, hi2(o[f]));
+        ql[f] = mul2(P, qxt, ol);
+        qh[f] = mul2(P, qxt, oh);
+        fl[f] = add2(Al[f], mul2(P, Wl[f], sub2(sub2(mul2(P, nq, nl), tl[f]), ql[f])));
+        fh[f] = add2(Ah[f], mul2(P, Wh[f], sub2(sub2(mul2(P, nq, nh), th[f]), qh[f])));
+    }
+    if (!LEFT) {
         // a chunk start (but the first) reads the value just computed for the column before it; the four
         // columns hold one at most, at the same place in every lane (x is a multiple of 4)
-        const int cs = (r0 - x) & 3;
-        const float pm = __shfl_up_sync(FULL, fh.y, 1, 16);
-        const float fn = cs == 0 ? pm : cs == 1 ? fl.x : cs == 2 ? fl.y : fh.x;
-        const float t = cs == 0 ? tl.x : cs == 1 ? tl.y : cs == 2 ? th.x : th.y;
-        const float q = cs == 0 ? ql.x : cs == 1 ? ql.y : cs == 2 ? qh.x : qh.y;
-        const float A = cs == 0 ? Al.x : cs == 1 ? Al.y : cs == 2 ? Ah.x : Ah.y;
-        const float W = cs == 0 ? Wl.x : cs == 1 ? Wl.y : cs == 2 ? Wh.x : Wh.y;
-        const float f = fadd(A, fmul(W, fsub(fsub(fmul(-P.qx, fn), t), q)));
-        const int i = x + cs;
+        const int cs = (r0 - x) & 3, i = x + cs;
         const bool start = i > r0 && ((i - r0) & 7) == 0;
-        if (start && cs == 0) fl.x = f;
-        if (start && cs == 1) fl.y = f;
-        if (start && cs == 2) fh.x = f;
-        if (start && cs == 3) fh.y = f;
-        if (row && x >= r0 && x <= P.nx - 2) n.x = fl.x;
-        if (row && x + 1 >= r0 && x + 1 <= P.nx - 2) n.y = fl.y;
-        if (row && x + 2 >= r0 && x + 2 <= P.nx - 2) n.z = fh.x;
-        if (row && x + 3 >= r0 && x + 3 <= P.nx - 2) n.w = fh.y;
+#pragma unroll
+        for (int f = 0; f < NF; ++f) {
+            const float pm = __shfl_up_sync(FULL, fh[f].y, 1, 16);
+            const float fn = cs == 0 ? pm : cs == 1 ? fl[f].x : cs == 2 ? fl[f].y : fh[f].x;
+            const float t = cs == 0 ? tl[f].x : cs == 1 ? tl[f].y : cs == 2 ? th[f].x : th[f].y;
+            const float q = cs == 0 ? ql[f].x : cs == 1 ? ql[f].y : cs == 2 ? qh[f].x : qh[f].y;
+            const float A = cs == 0 ? Al[f].x : cs == 1 ? Al[f].y : cs == 2 ? Ah[f].x : Ah[f].y;
+            const float W = cs == 0 ? Wl[f].x : cs == 1 ? Wl[f].y : cs == 2 ? Wh[f].x : Wh[f].y;
+            const float g = fadd(A, fmul(W, fsub(fsub(fmul(-P.qx, fn), t), q)));
+            if (start && cs == 0) fl[f].x = g;
+            if (start && cs == 1) fl[f].y = g;
+            if (start && cs == 2) fh[f].x = g;
+            if (start && cs == 3) fh[f].y = g;
+        }
     }
+#pragma unroll
+    for (int f = 0; f < NF; ++f) {
+        if (m[0]) n[f].x = fl[f].x;
+        if (m[1]) n[f].y = fl[f].y;
+        if (m[2]) n[f].z = fh[f].x;
+        if (m[3]) n[f].w = fh[f].y;
+    }
+}
+
+template <int NF>
+__device__ __forceinline__ void side_rules(const StepParams& P, bool left, bool right, const float4 (&w)[NF], int x, int j,
+                                           float4 (&n)[NF], const float4 (&o)[NF]) {
+    float4 pre[NF];
+#pragma unroll
+    for (int f = 0; f < NF; ++f) pre[f] = n[f];
+    if (left) side_band<NF, true>(P, w, x, j, pre, o, n);
+    if (right) side_band<NF, false>(P, w, x, j, pre, o, n);
 }
 
 // Weights of columns x..x+3 of row j from a table by distance.  Below the
@@ -547,8 +574,10 @@ static __device__ __noinline__ float4 side_rules_call(SideParams S, const float*
     P.qt_x = S.qt_x;
     P.qxt = S.qxt;
     P.neg_zero = S.neg_zero;
-    side_rules(P, left, right, side_weights(P, tab, x, j), x, j, n, o);
-    return n;
+    const float4 w[1] = {side_weights(P, tab, x, j)}, oa[1] = {o};
+    float4 na[1] = {n};
+    side_rules(P, left, right, w, x, j, na, oa);
+    return na[0];
 }
 
 

@@ -72,6 +72,8 @@ int main() {
             const size_t need = sizeof(float) * resident_smem_floats(M, b, h, r == L.rows - 1, r == 0 && !fs, false, iso);
             rule(need <= p.smem && p.smem == sizeof(float) * (size_t)L.smem_floats && p.smem <= 227 * 1024 - 256, "shared memory", nx, nz, M, b, fs);
         }
+        rule(nx - 2 * b - 1 >= 4, "no four columns of both side bands", nx, nz, M, b, fs);
+        rule(resident_plane(M, L.h_max) < 65536, "plane offsets in 16 bits", nx, nz, M, b, fs);
         rule(L.x_edge[1] >= b + 2, "left band and the column after it in the first strip", nx, nz, M, b, fs);
         rule(L.x_edge[L.strips - 1] <= nx - b - 2, "right band and the column before it in the last strip", nx, nz, M, b, fs);
         rule(L.z_edge[L.rows - 1] <= nz - b - 2, "bottom band and the row above it in the last row", nx, nz, M, b, fs);
