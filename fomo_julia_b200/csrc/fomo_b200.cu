@@ -743,7 +743,7 @@ std::mutex g_step_choice_mu;
 std::map<StepKey, int> g_step_choice;
 constexpr int kStepTuneWindow = 24;  // steps timed per candidate
 
-// The autotuners' optional cache file (environment variable
+// The optional cache file of step-kernel choices (environment variable
 // FOMO_B200_TUNE_CACHE).  Single-shot kernel choices are lines
 // "step nx nz M nbc fs iso choice", read on first use and appended to when a
 // choice is made; the shot server's lines have five numbers (server.cuh).

@@ -118,10 +118,24 @@ struct Request {
     cudaEvent_t done_ev = nullptr;
 };
 
-// K candidates of the autotuner: 1 = plain launches (chunks of kPlainChunk
+// Time steps per launch a batch can be told to run (a cache file's choice or
+// the server's configuration): 1 = plain launches (chunks of kPlainChunk
 // steps), otherwise one graph of K steps.
-constexpr int kTuneK[3] = {1, 8, 32};
+constexpr int kStepChoices[3] = {1, 8, 32};
+// What a batch runs otherwise: graphs of 8 steps.  A replay costs a few
+// microseconds, a rebuild of the graph about 0.1 ms a step, and the graphs are
+// rebuilt whenever a shot joins or leaves.  Over batches of 1 to 30 shots on
+// grids from 208 x 128 to 4552 x 3927, graphs of 8 steps were the fastest or
+// within 1% of it (16 shots on 2108 x 908, nt 400: 135 ms at 8, 138 at 32, 161
+// at 128), and timing candidates on live chunks, as the server used to, chose
+// wrong often enough to cost more than it gained.
+constexpr int kStepsDefault = 1;  // index in kStepChoices
 constexpr int kPlainChunk = 32;
+// Chains of launches side by side (enqueue_steps).  One, two and four chains:
+// 24 shots on 508 x 308, nt 800, 72, 59 and 58 ms; 30 on 208 x 128, nt 2000,
+// 150, 121 and 83; 20 on mixed media 134, 131 and 132; no difference where one
+// set fills the device.
+constexpr int kChains = 4;
 constexpr int kMaxInFlight = 4096;  // shots in flight per server (launch sets <= shots)
 
 struct TuneKey {
@@ -130,21 +144,8 @@ struct TuneKey {
         return std::tie(nx, nz, M, shots_log2) < std::tie(o.nx, o.nz, o.M, o.shots_log2);
     }
 };
-constexpr int kTuneSamples = 2;  // chunks timed per candidate (the fastest counts)
-// Candidates the autotuner times: graphs of 8 and of 32 steps.  Plain
-// launches (kTuneK[0]) run only when configured: over the bench's batched,
-// uneven and serving runs the tuner never chose them, and their timed chunks
-// are the slowest of a short mixed run.
-constexpr int kTuneFirst = 1;
-struct TuneEntry {
-    // device time per cell-step of the shots in flight (ms per Gcell-step):
-    // comparable across chunks whose shots differ; the lowest of the samples
-    double ms_per_work[3] = {-1, -1, -1};
-    int samples[3] = {0, 0, 0};
-    int chosen = -1;
-};
 std::mutex g_tune_mu;
-std::map<TuneKey, TuneEntry> g_tune;  // process-wide cache: (grid, order, batch size) -> K
+std::map<TuneKey, int> g_tune;  // process-wide: (grid, order, batch size) -> index in kStepChoices
 
 // Optional file behind the cache (environment variable FOMO_B200_TUNE_CACHE,
 // tune_cache_path): one line "nx nz M shots_log2 K" per decision, read when a
@@ -161,7 +162,7 @@ void load_tune_cache() {
     while (std::fgets(line, sizeof(line), f))
         if (std::sscanf(line, "%d %d %d %d %d", &nx, &nz, &M, &lg, &K) == 5)
             for (int c = 0; c < 3; ++c)
-                if (kTuneK[c] == K) g_tune[TuneKey{nx, nz, M, lg}].chosen = c;
+                if (kStepChoices[c] == K) g_tune[TuneKey{nx, nz, M, lg}] = c;
     std::fclose(f);
 }
 
@@ -169,7 +170,7 @@ void save_tune_choice(const TuneKey& k, int cand) {
     const char* path = tune_cache_path();
     if (!path) return;
     if (FILE* f = std::fopen(path, "a")) {
-        std::fprintf(f, "%d %d %d %d %d\n", k.nx, k.nz, k.M, k.shots_log2, kTuneK[cand]);
+        std::fprintf(f, "%d %d %d %d %d\n", k.nx, k.nz, k.M, k.shots_log2, kStepChoices[cand]);
         std::fclose(f);
     }
 }
@@ -300,24 +301,24 @@ bool march_ok(const Request& r) {
 // A set's tile launch of one half step (after_band: a dependent launch
 // beside the band pass just before it, see launch_tiles).
 template <int M>
-void launch_batch_M(bool vel, const LaunchSet& S, cudaStream_t st, bool after_band) {
+cudaError_t launch_batch_M(bool vel, const LaunchSet& S, cudaStream_t st, bool after_band) {
     if (vel)
-        launch_tiles(S.gen ? fomo::batch_velocity_kernel<M, true> : fomo::batch_velocity_kernel<M, false>, S.grid_v, S.smem_v, st,
+        return launch_tiles(S.gen ? fomo::batch_velocity_kernel<M, true> : fomo::batch_velocity_kernel<M, false>, S.grid_v, S.smem_v, st,
                      after_band, *S.lv);
-    else
-        launch_tiles(S.gen ? fomo::batch_stress_kernel<M, true> : fomo::batch_stress_kernel<M, false>, S.grid_s, S.smem_s, st,
-                     after_band, *S.ls);
+    return launch_tiles(S.gen ? fomo::batch_stress_kernel<M, true> : fomo::batch_stress_kernel<M, false>, S.grid_s, S.smem_s, st,
+                        after_band, *S.ls);
 }
 
-void launch_batch(bool vel, const LaunchSet& S, cudaStream_t st, bool after_band) {
+cudaError_t launch_batch(bool vel, const LaunchSet& S, cudaStream_t st, bool after_band) {
     switch (S.M) {
-        case 1: launch_batch_M<1>(vel, S, st, after_band); break;
-        case 2: launch_batch_M<2>(vel, S, st, after_band); break;
-        case 3: launch_batch_M<3>(vel, S, st, after_band); break;
-        case 4: launch_batch_M<4>(vel, S, st, after_band); break;
-        case 5: launch_batch_M<5>(vel, S, st, after_band); break;
-        case 6: launch_batch_M<6>(vel, S, st, after_band); break;
+        case 1: return launch_batch_M<1>(vel, S, st, after_band);
+        case 2: return launch_batch_M<2>(vel, S, st, after_band);
+        case 3: return launch_batch_M<3>(vel, S, st, after_band);
+        case 4: return launch_batch_M<4>(vel, S, st, after_band);
+        case 5: return launch_batch_M<5>(vel, S, st, after_band);
+        case 6: return launch_batch_M<6>(vel, S, st, after_band);
     }
+    return cudaErrorInvalidValue;
 }
 
 class Server {
@@ -328,6 +329,7 @@ class Server {
         device_ = device;
         CUDA_TRY(cudaSetDevice(device));
         CUDA_TRY(cudaStreamCreateWithFlags(&st_, cudaStreamNonBlocking));
+        for (auto& q : aux_) CUDA_TRY(cudaStreamCreateWithFlags(&q, cudaStreamNonBlocking));
         cudaMemPoolProps props;
         std::memset(&props, 0, sizeof(props));
         props.allocType = cudaMemAllocationTypePinned;
@@ -379,13 +381,15 @@ class Server {
         deferred_.clear();
         for (auto e : ev_free_) cudaEventDestroy(e);
         ev_free_.clear();
-        for (auto e : tev_free_) cudaEventDestroy(e);
-        tev_free_.clear();
         if (st_) cudaStreamSynchronize(st_);
         if (d_ctl_) cudaFree(d_ctl_);
         d_ctl_ = nullptr;
         if (pool_) cudaMemPoolDestroy(pool_);
         pool_ = nullptr;
+        for (auto& q : aux_) {
+            if (q) cudaStreamDestroy(q);
+            q = nullptr;
+        }
         if (st_) cudaStreamDestroy(st_);
         st_ = nullptr;
         std::lock_guard<std::mutex> lk(mu_);
@@ -473,17 +477,11 @@ class Server {
         cudaGraphExec_t exec = nullptr;
         void* pinned = nullptr;
     };
-    struct Measure {   // a timed chunk of the autotuner
-        TuneKey key;
-        int cand;
-        double work;     // Gcell-steps of the chunk: steps x cells of the shots in flight
-        cudaEvent_t a, b;
-    };
-
     FomoServerConfig cfg_;
     int device_ = 0;
     size_t budget_ = 0;
     cudaStream_t st_ = nullptr;
+    cudaStream_t aux_[kChains - 1] = {};  // the further chains' streams, idle between chunks
     cudaMemPool_t pool_ = nullptr;
     unsigned char* d_ctl_ = nullptr;
     int* d_counters_ = nullptr;   // per launch set: velocity and stress batch step
@@ -512,23 +510,21 @@ class Server {
     std::map<int, cudaGraphExec_t> graphs_;  // 2K + parity of its first step -> graph of the current tables
     std::deque<cudaEvent_t> inflight_;
     std::vector<Deferred> deferred_;
-    std::vector<Measure> measures_;
-    std::vector<cudaEvent_t> ev_free_, tev_free_;
+    std::vector<cudaEvent_t> ev_free_;
     PinnedPool pinned_;
 
     // ------------------------------------------------------------ helpers
-    cudaEvent_t event(bool timing = false) {
-        auto& fl = timing ? tev_free_ : ev_free_;
-        if (!fl.empty()) {
-            cudaEvent_t e = fl.back();
-            fl.pop_back();
+    cudaEvent_t event() {
+        if (!ev_free_.empty()) {
+            cudaEvent_t e = ev_free_.back();
+            ev_free_.pop_back();
             return e;
         }
         cudaEvent_t e = nullptr;
-        cudaEventCreateWithFlags(&e, timing ? cudaEventDefault : cudaEventDisableTiming);
+        cudaEventCreateWithFlags(&e, cudaEventDisableTiming);
         return e;
     }
-    void release_event(cudaEvent_t e, bool timing = false) { (timing ? tev_free_ : ev_free_).push_back(e); }
+    void release_event(cudaEvent_t e) { ev_free_.push_back(e); }
 
     static std::tuple<Medium*, uint32_t, uint32_t> res_key(const Request& r) {
         uint32_t bx, bz;
@@ -791,6 +787,11 @@ class Server {
         // One launch set per run of at most kShotsPerLaunch shots with the
         // same M; everything it needs goes into its kernel parameters.
         for (size_t i = 0; i < order.size();) {
+            // the shots of an FD order in sets of equal size, so that the chains are as long as each other
+            size_t run = i;
+            while (run < order.size() && order[run]->M == order[i]->M) ++run;
+            const size_t left = run - i, n_sets = (left + fomo::kShotsPerLaunch - 1) / fomo::kShotsPerLaunch;
+            const size_t cap = (left + n_sets - 1) / n_sets;
             LaunchSet S;
             S.M = order[i]->M;
             S.lv = std::make_shared<fomo::BatchVelLaunch>();
@@ -801,11 +802,9 @@ class Server {
             int band = 0, tile = 0, n_groups = 0;
             size_t j = i;
             while (j < order.size() && order[j]->M == S.M && n_groups < fomo::kMaxGroups &&
-                   j - i < (size_t)fomo::kShotsPerLaunch) {
+                   j - i < cap) {
                 size_t h = j;
-                while (h < order.size() && order[h]->M == S.M && order[h]->med == order[j]->med &&
-                       h - i < (size_t)fomo::kShotsPerLaunch)
-                    ++h;
+                while (h < order.size() && order[h]->M == S.M && order[h]->med == order[j]->med && h - i < cap) ++h;
                 const Launch L = shape_of(*order[j]);
                 fomo::GroupDev& G = H.groups[n_groups++];
                 G.first = (int)(j - i);
@@ -955,33 +954,58 @@ class Server {
     // ------------------------------------------------------------ stepping
     int launches_per_step() const { return 4 * (int)sets_.size() + (int)msets_.size(); }
 
-    // One batch step, set after set.  `after_band`: the last launch on the
-    // stream is the previous step's last stress band pass, so the first
-    // velocity launch may start beside it (every later tile launch follows
-    // a band pass).  `k`: the batch step (only its parity goes into the
-    // launches, which take it as the copy parity of their shots).
-    void enqueue_step(bool after_band, int64_t k) {
-        // the previous step ended with a band pass only without fused-step sets
-        after_band = after_band && msets_.empty();
-        for (size_t i = 0; i < sets_.size(); ++i) {
-            const LaunchSet& S = sets_[i];
-            S.lv->H.kpar = S.ls->H.kpar = (int)(k & 1);
-            launch_batch(true, S, st_, after_band || i > 0);
-            fomo::batch_band_kernel<true, fomo::BatchVelLaunch><<<S.grid_b, 32, 0, st_>>>(*S.lv);
-            launch_batch(false, S, st_, true);
-            fomo::batch_band_kernel<false, fomo::BatchStrLaunch><<<S.grid_b, 32, 0, st_>>>(*S.ls);
+    // `n` batch steps from step `k0` (only a step's parity goes into the
+    // launches, which take it as the copy parity of their shots).  The launch
+    // sets are independent of each other: they run in up to kChains chains of
+    // launches side by side, set i in chain i % chains, so that one set's
+    // band passes and last waves of tiles are filled by another's tiles.
+    // Inside a chain every tile launch but the first follows a band pass on
+    // its stream and may start beside it.  The chains fork from the server's
+    // stream and join it again (in a captured graph these are its branches).
+    void enqueue_steps(int n, int64_t k0) {
+        const int chains = std::max(1, std::min<int>(kChains, (int)sets_.size()));
+        cudaStream_t st[kChains] = {st_};
+        if (chains > 1) {
+            cudaEvent_t fork = event();
+            note(cudaEventRecord(fork, st_));
+            for (int c = 1; c < chains; ++c) {
+                st[c] = aux_[c - 1];
+                note(cudaStreamWaitEvent(st[c], fork, 0));
+            }
+            release_event(fork);
         }
-        for (const MarchSet& S : msets_) {
-            const cudaError_t e = batch_march_launch_any(S.M, S.grid, st_, *S.L);
-            if (e != cudaSuccess && enqueue_err_ == cudaSuccess) enqueue_err_ = e;
+        for (int k = 0; k < n; ++k) {
+            for (size_t i = 0; i < sets_.size(); ++i) {
+                const LaunchSet& S = sets_[i];
+                cudaStream_t q = st[i % chains];
+                // the step before ended with a band pass on the chain's stream, unless fused-step sets ran after it
+                const bool after_band = (k > 0 && (msets_.empty() || i % chains > 0)) || i >= (size_t)chains;
+                S.lv->H.kpar = S.ls->H.kpar = (int)((k0 + k) & 1);
+                note(launch_batch(true, S, q, after_band));
+                fomo::batch_band_kernel<true, fomo::BatchVelLaunch><<<S.grid_b, 32, 0, q>>>(*S.lv);
+                note(launch_batch(false, S, q, true));
+                fomo::batch_band_kernel<false, fomo::BatchStrLaunch><<<S.grid_b, 32, 0, q>>>(*S.ls);
+            }
+            for (const MarchSet& S : msets_) note(batch_march_launch_any(S.M, S.grid, st_, *S.L));
+        }
+        for (int c = 1; c < chains; ++c) {
+            cudaEvent_t join = event();
+            note(cudaEventRecord(join, st[c]));
+            note(cudaStreamWaitEvent(st_, join, 0));
+            release_event(join);
         }
     }
 
-    // The first launch error of the fused-step sets since the last check.
+    // Keeps the first error of the launches enqueued since the last check.
+    void note(cudaError_t e) {
+        if (e != cudaSuccess && enqueue_err_ == cudaSuccess) enqueue_err_ = e;
+    }
+
+    // The first launch error since the last check.
     int take_enqueue_error() {
         const cudaError_t e = enqueue_err_;
         enqueue_err_ = cudaSuccess;
-        if (e != cudaSuccess) return fail(FOMO_ECUDA, "fused-step batch launch failed: %s", cudaGetErrorString(e));
+        if (e != cudaSuccess) return fail(FOMO_ECUDA, "batch launch failed: %s", cudaGetErrorString(e));
         return FOMO_OK;
     }
 
@@ -995,7 +1019,7 @@ class Server {
         }
         cudaGraph_t g = nullptr;
         CUDA_TRY(cudaStreamBeginCapture(st_, cudaStreamCaptureModeThreadLocal));
-        for (int k = 0; k < K; ++k) enqueue_step(k > 0, p0 + k);
+        enqueue_steps(K, p0);
         cudaError_t e = cudaStreamEndCapture(st_, &g);
         if (int rc = take_enqueue_error()) {
             if (g) cudaGraphDestroy(g);
@@ -1006,7 +1030,7 @@ class Server {
         e = cudaGraphInstantiate(&x, g, 0);
         cudaGraphDestroy(g);
         if (e != cudaSuccess) return fail(FOMO_ECUDA, "graph instantiation failed: %s", cudaGetErrorString(e));
-        // upload now, so the first replay (maybe a timed one) does not carry it
+        // upload now, so that the first replay does not carry it
         e = cudaGraphUpload(x, st_);
         if (e != cudaSuccess) return fail(FOMO_ECUDA, "graph upload failed: %s", cudaGetErrorString(e));
         graphs_[key] = x;
@@ -1024,103 +1048,42 @@ class Server {
         return TuneKey{big->med->nx, big->med->nz, big->M, lg};
     }
 
-    // Candidate index of the next chunk: the cached choice, else the first
-    // candidate neither measured nor being measured for this key.
-    int choose(const TuneKey& key, bool* measure) {
-        *measure = false;
+    // Index in kStepChoices of the next chunk (-2: a configured K that is none
+    // of them): the configuration's, the cache file's, or the default, which
+    // is entered in the cache.
+    int choose(const TuneKey& key) {
         if (cfg_.steps_per_launch > 0) {
             for (int c = 0; c < 3; ++c)
-                if (kTuneK[c] == cfg_.steps_per_launch) return c;
-            return -2;  // a K outside the candidates: graphs of exactly that K
+                if (kStepChoices[c] == cfg_.steps_per_launch) return c;
+            return -2;
         }
         std::lock_guard<std::mutex> lk(g_tune_mu);
-        TuneEntry& e = g_tune[key];
-        if (e.chosen >= 0) return e.chosen;
-        for (int c = kTuneFirst; c < 3; ++c)
-            if (e.samples[c] < kTuneSamples) {
-                bool pending = false;
-                for (auto& m : measures_)
-                    if (!(m.key < key) && !(key < m.key) && m.cand == c) pending = true;
-                if (!pending) {
-                    *measure = true;
-                    return c;
-                }
-            }
-        return 1;  // all measured or pending: K = 8 meanwhile
-    }
-
-    void resolve_measures(bool block) {
-        for (size_t i = 0; i < measures_.size();) {
-            Measure& m = measures_[i];
-            if (block) cudaEventSynchronize(m.b);
-            if (cudaEventQuery(m.b) != cudaSuccess) {
-                ++i;
-                continue;
-            }
-            float ms = 0;
-            cudaEventElapsedTime(&ms, m.a, m.b);
-            {
-                std::lock_guard<std::mutex> lk(g_tune_mu);
-                TuneEntry& e = g_tune[m.key];
-                const double t = ms / m.work;
-                if (e.ms_per_work[m.cand] < 0 || t < e.ms_per_work[m.cand]) e.ms_per_work[m.cand] = t;
-                e.samples[m.cand] += 1;
-                bool all = true;
-                int best = kTuneFirst;
-                for (int c = kTuneFirst; c < 3; ++c) {
-                    if (e.samples[c] < kTuneSamples) all = false;
-                    if (e.ms_per_work[c] >= 0 && (e.ms_per_work[best] < 0 || e.ms_per_work[c] < e.ms_per_work[best])) best = c;
-                }
-                if (all && e.chosen < 0) {
-                    e.chosen = best;
-                    save_tune_choice(m.key, best);
-                }
-            }
-            release_event(m.a, true);
-            release_event(m.b, true);
-            measures_.erase(measures_.begin() + i);
-        }
+        const auto [it, added] = g_tune.emplace(key, kStepsDefault);
+        if (added) save_tune_choice(key, it->second);
+        return it->second;
     }
 
     int run_chunk() {
         int64_t rem = INT64_MAX;
         for (auto& r : active_) rem = std::min<int64_t>(rem, (int64_t)r->start + r->nt - 1 - k_host_);
-        const TuneKey key = tune_key();
-        bool measure = false;
-        const int cand = choose(key, &measure);
-        const int K = cand >= 0 ? kTuneK[cand] : cfg_.steps_per_launch;
+        const int cand = choose(tune_key());
+        const int K = cand >= 0 ? kStepChoices[cand] : cfg_.steps_per_launch;
         const int chunk = K == 1 ? kPlainChunk : K;
         const int n = (int)std::min<int64_t>(chunk, rem);
         const bool graph = K > 1 && n == K;
-        if (n != chunk) measure = false;
         cudaGraphExec_t x = nullptr;
         if (graph)
             if (int rc = graph_for(K, (int)((k_host_ + 1) & 1), &x)) return rc;
-        Measure ms{};
-        if (measure) {
-            double cells = 0;
-            for (auto& r : active_) cells += (double)r->med->nx * r->med->nz;
-            ms.key = key;
-            ms.cand = cand;
-            ms.work = n * cells / 1e9;
-            ms.a = event(true);
-            ms.b = event(true);
-            CUDA_TRY(cudaEventRecord(ms.a, st_));
-        }
         nvtxRangePushA(graph ? "fomo_b200 batch graph replay" : "fomo_b200 batch launches");
         if (graph) {
             const cudaError_t e = cudaGraphLaunch(x, st_);
             nvtxRangePop();
             CUDA_TRY(e);
         } else {
-            for (int k = 0; k < n; ++k) enqueue_step(k > 0, k_host_ + 1 + k);
+            enqueue_steps(n, k_host_ + 1);
             nvtxRangePop();
             CUDA_TRY(cudaGetLastError());
             if (int rc = take_enqueue_error()) return rc;
-        }
-        if (measure) {
-            CUDA_TRY(cudaEventRecord(ms.b, st_));
-            measures_.push_back(ms);
         }
         k_host_ += n;
         {
@@ -1244,7 +1207,6 @@ class Server {
         while (true) {
             complete_retired(false);
             release_deferred(false);
-            resolve_measures(false);
             std::vector<std::shared_ptr<Request>> admitted;
             {
                 std::unique_lock<std::mutex> lk(mu_);
@@ -1339,7 +1301,6 @@ class Server {
             release_event(e);
         }
         inflight_.clear();
-        resolve_measures(true);
         release_deferred(true);
     }
 };
