@@ -68,6 +68,7 @@ struct Buffer : Object {
 // and no device-wide synchronisation (cudaFree has both).
 cudaError_t pool_alloc(void** p, size_t bytes);
 void pool_free(void* p);
+void trim_server_pool(size_t keep);  // server.cuh
 
 // Row pitch in floats: rows start on 128-byte boundaries.
 inline int pitch_of(int nx) { return (nx + 31) / 32 * 32; }
@@ -143,9 +144,15 @@ struct Context {
     ulonglong2* mail = nullptr;  // mailboxes of the resident kernel, and their number of messages
     size_t mail_items = 0;
     uint32_t mail_tag = 1;       // tag of the next resident step (0: never sent)
+    unsigned char* pinned = nullptr;  // host staging of small read-backs (kPinnedBytes), the status word first
     uint64_t next = 1;
     std::unordered_map<uint64_t, std::unique_ptr<Object>> objs;
 };
+
+// Read-backs up to this size go through pinned memory: a frame or gather of a
+// few hundred KB otherwise waits for the driver's own staging of pageable
+// memory (a 554 x 254 frame: 143 -> 80 us with its kernel).
+constexpr size_t kPinnedBytes = 4 << 20, kPinnedHead = 256;
 
 Context& ctx() {
     static Context c;
@@ -159,6 +166,7 @@ cudaError_t pool_alloc(void** p, size_t bytes) {
         (void)cudaGetLastError();
         cudaStreamSynchronize(C.stream);
         cudaMemPoolTrimTo(C.pool, 0);
+        trim_server_pool(0);
         e = cudaMallocFromPoolAsync(p, bytes, C.pool, C.stream);
     }
     if (e != cudaSuccess) {
@@ -401,14 +409,43 @@ struct Profile {
     }
 };
 
+// Copies `bytes` from the device to `host` on the library stream and waits.
+int read_back(void* host, const void* dev, size_t bytes) {
+    auto& C = ctx();
+    if (!C.pinned || bytes > kPinnedBytes - kPinnedHead) {
+        CUDA_TRY(cudaMemcpyAsync(host, dev, bytes, cudaMemcpyDeviceToHost, C.stream));
+        CUDA_TRY(cudaStreamSynchronize(C.stream));
+        return FOMO_OK;
+    }
+    CUDA_TRY(cudaMemcpyAsync(C.pinned + kPinnedHead, dev, bytes, cudaMemcpyDeviceToHost, C.stream));
+    CUDA_TRY(cudaStreamSynchronize(C.stream));
+    std::memcpy(host, C.pinned + kPinnedHead, bytes);
+    return FOMO_OK;
+}
+
+// The end of a run of steps: waits for it, adds its device time to the shot
+// and reports the kernels' status word.
+int finish_steps(Shot& s);
+
 int check_status() {
     int st = 0;
-    CUDA_TRY(cudaMemcpyAsync(&st, ctx().d_status, sizeof(int), cudaMemcpyDeviceToHost, ctx().stream));
-    CUDA_TRY(cudaStreamSynchronize(ctx().stream));
+    auto& C = ctx();
+    int* h = C.pinned ? reinterpret_cast<int*>(C.pinned) : &st;
+    CUDA_TRY(cudaMemcpyAsync(h, C.d_status, sizeof(int), cudaMemcpyDeviceToHost, C.stream));
+    CUDA_TRY(cudaStreamSynchronize(C.stream));
+    st = *h;
     if (st == fomo::kErrTmaTimeout) return fail(FOMO_ETIMEOUT, "a TMA load of a time-step kernel did not complete");
     if (st == fomo::kErrResidentTimeout) return fail(FOMO_ETIMEOUT, "a block of the resident kernel did not hear from its neighbours");
     if (st) return fail(FOMO_ECUDA, "time-step kernel reported error %d", st);
     return FOMO_OK;
+}
+
+int finish_steps(Shot& s) {
+    const int rc = check_status();  // waits for the stream, and so for ev1
+    float ms = 0;
+    CUDA_TRY(cudaEventElapsedTime(&ms, ctx().ev0, ctx().ev1));
+    s.device_ms += ms;
+    return rc;
 }
 
 // Launches a tile kernel.  With `after_band` (the launch just before it on
@@ -594,11 +631,7 @@ int run_steps_march(Shot& s, Medium& m, Wavefield& w, int n_steps, Profile* prof
     nvtxRangePop();
     CUDA_TRY(cudaGetLastError());
     CUDA_TRY(cudaEventRecord(C.ev1, C.stream));
-    CUDA_TRY(cudaEventSynchronize(C.ev1));
-    float ms = 0;
-    CUDA_TRY(cudaEventElapsedTime(&ms, C.ev0, C.ev1));
-    s.device_ms += ms;
-    return check_status();
+    return finish_steps(s);
 }
 
 // ---------------------------------------------------------------- resident steps
@@ -676,11 +709,7 @@ int run_steps_resident(Shot& s, Medium& m, Wavefield& w, int n_steps, const fomo
     }
     nvtxRangePop();
     CUDA_TRY(cudaEventRecord(C.ev1, C.stream));
-    CUDA_TRY(cudaEventSynchronize(C.ev1));
-    float ms = 0;
-    CUDA_TRY(cudaEventElapsedTime(&ms, C.ev0, C.ev1));
-    s.device_ms += ms;
-    return check_status();
+    return finish_steps(s);
 }
 
 // The fused step's plan for a shot, or !ok (split launches): FOMO_STEP_SPLIT,
@@ -895,11 +924,7 @@ int run_steps_split(Shot& s, Medium& m, Wavefield& w, int n_steps, Profile* prof
     nvtxRangePop();
     CUDA_TRY(cudaGetLastError());
     CUDA_TRY(cudaEventRecord(C.ev1, C.stream));
-    CUDA_TRY(cudaEventSynchronize(C.ev1));
-    float ms = 0;
-    CUDA_TRY(cudaEventElapsedTime(&ms, C.ev0, C.ev1));
-    s.device_ms += ms;
-    return check_status();
+    return finish_steps(s);
 }
 
 int run_steps(Shot& s, int n_steps, Profile* prof = nullptr) {
@@ -919,6 +944,7 @@ int run_steps(Shot& s, int n_steps, Profile* prof = nullptr) {
 
 // Records the receivers of the last step done (the next velocity launch would).
 void shutdown_servers();  // server.cuh
+void destroy_server_pool();
 
 int record_last(Shot& s) {
     auto& C = ctx();
@@ -973,6 +999,10 @@ int fomo_b200_init(int device) {
     CUDA_TRY(cudaMemPoolCreate(&C.pool, &props));
     uint64_t keep = UINT64_MAX;
     CUDA_TRY(cudaMemPoolSetAttribute(C.pool, cudaMemPoolAttrReleaseThreshold, &keep));
+    if (cudaHostAlloc((void**)&C.pinned, kPinnedBytes, cudaHostAllocDefault) != cudaSuccess) {
+        (void)cudaGetLastError();  // read-backs go straight to the caller's memory
+        C.pinned = nullptr;
+    }
     C.device = device;
     C.inited = true;
     return FOMO_OK;
@@ -980,6 +1010,7 @@ int fomo_b200_init(int device) {
 
 int fomo_b200_shutdown(void) {
     shutdown_servers();
+    destroy_server_pool();
     auto& C = ctx();
     std::lock_guard<std::mutex> lk(C.mu);
     if (!C.inited) return FOMO_OK;
@@ -995,6 +1026,8 @@ int fomo_b200_shutdown(void) {
     cudaEventDestroy(C.ev1);
     cudaFree(C.d_status);
     C.d_status = nullptr;
+    if (C.pinned) cudaFreeHost(C.pinned);
+    C.pinned = nullptr;
     cudaStreamDestroy(C.stream);
     C.stream = nullptr;
     C.inited = false;
@@ -1267,9 +1300,7 @@ int fomo_b200_wavefield_snapshot(uint64_t wavefield, int32_t kind, int32_t downs
     fomo::snapshot_kernel<<<4 * sm_count(), 256, 0, ctx().stream>>>(f0, f1, kind, w->nx, w->nz, w->pitch, downsample, nx_d,
                                                              nz_d, w->snap);
     CUDA_TRY(cudaGetLastError());
-    CUDA_TRY(cudaMemcpyAsync(host, w->snap, bytes, cudaMemcpyDeviceToHost, ctx().stream));
-    CUDA_TRY(cudaStreamSynchronize(ctx().stream));
-    return FOMO_OK;
+    return read_back(host, w->snap, bytes);
 }
 
 // ---------------------------------------------------------------- shots
@@ -1389,7 +1420,7 @@ int fomo_b200_shot_finish(uint64_t shot_handle, float* gather_out, FomoRunStats*
     if (int rc = record_last(*s)) return rc;
     if (gather_out && s->n_rec && s->nt) {
         const size_t bytes = (size_t)s->nt * s->n_rec * sizeof(float);
-        CUDA_TRY(cudaMemcpyAsync(gather_out, s->d_gather, bytes, cudaMemcpyDeviceToHost, ctx().stream));
+        if (int rc = read_back(gather_out, s->d_gather, bytes)) return rc;
         s->d2h += bytes;
     }
     CUDA_TRY(cudaStreamSynchronize(ctx().stream));

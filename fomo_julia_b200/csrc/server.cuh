@@ -3,8 +3,8 @@
 // Part of fomo_b200.cu's translation unit (included after the runtime's
 // internals: fail, ctx, Medium, encode_map, Launch, ...).
 //
-// One worker thread per server owns a CUDA stream, a stream-ordered memory
-// pool and the batch loop:
+// One worker thread per server owns the CUDA streams of its launches and the
+// batch loop; the servers' shots share one stream-ordered memory pool:
 //   admit   queued requests, in arrival order, while their device bytes fit
 //           the HBM budget (and the shot limit); allocate and upload each
 //           shot, starting it at the next batch step;
@@ -321,6 +321,72 @@ cudaError_t launch_batch(bool vel, const LaunchSet& S, cudaStream_t st, bool aft
     return cudaErrorInvalidValue;
 }
 
+// Device memory of the servers' shots: one stream-ordered pool for all of
+// them, kept between servers (fomo_b200_run_batch makes one for each call, and
+// mapping a batch's memory anew took 7-20 ms of it, many times that on some
+// hosts).  What is freed stays mapped while a server lives; once the last one
+// is gone kServerPoolKeep bytes stay, until the library needs the memory or
+// shuts down.  The pool orders reuse across the servers' streams itself.
+constexpr size_t kServerPoolKeep = 2ull << 30;
+struct ServerPool {
+    std::mutex mu;
+    cudaMemPool_t pool = nullptr;
+    int servers = 0;
+};
+ServerPool& server_pool() {
+    static ServerPool p;
+    return p;
+}
+
+int acquire_server_pool(int device, cudaMemPool_t* out) {
+    auto& S = server_pool();
+    std::lock_guard<std::mutex> lk(S.mu);
+    if (!S.pool) {
+        cudaMemPoolProps props;
+        std::memset(&props, 0, sizeof(props));
+        props.allocType = cudaMemAllocationTypePinned;
+        props.handleTypes = cudaMemHandleTypeNone;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = device;
+        CUDA_TRY(cudaMemPoolCreate(&S.pool, &props));
+        uint64_t keep = UINT64_MAX;
+        CUDA_TRY(cudaMemPoolSetAttribute(S.pool, cudaMemPoolAttrReleaseThreshold, &keep));
+    }
+    S.servers += 1;
+    *out = S.pool;
+    return FOMO_OK;
+}
+
+void release_server_pool() {
+    auto& S = server_pool();
+    std::lock_guard<std::mutex> lk(S.mu);
+    if (--S.servers == 0) cudaMemPoolTrimTo(S.pool, kServerPoolKeep);
+}
+
+void trim_server_pool(size_t keep) {
+    auto& S = server_pool();
+    std::lock_guard<std::mutex> lk(S.mu);
+    if (S.pool) cudaMemPoolTrimTo(S.pool, keep);
+}
+
+// Mapped and unused bytes of the pool: a new server can have them too.
+size_t server_pool_cached() {
+    auto& S = server_pool();
+    std::lock_guard<std::mutex> lk(S.mu);
+    uint64_t reserved = 0, used = 0;
+    if (!S.pool || cudaMemPoolGetAttribute(S.pool, cudaMemPoolAttrReservedMemCurrent, &reserved) != cudaSuccess ||
+        cudaMemPoolGetAttribute(S.pool, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess)
+        return 0;
+    return reserved > used ? (size_t)(reserved - used) : 0;
+}
+
+void destroy_server_pool() {  // no server is left
+    auto& S = server_pool();
+    std::lock_guard<std::mutex> lk(S.mu);
+    if (S.pool) cudaMemPoolDestroy(S.pool);
+    S.pool = nullptr;
+}
+
 class Server {
   public:
     explicit Server(const FomoServerConfig& cfg) : cfg_(cfg) {}
@@ -330,15 +396,7 @@ class Server {
         CUDA_TRY(cudaSetDevice(device));
         CUDA_TRY(cudaStreamCreateWithFlags(&st_, cudaStreamNonBlocking));
         for (auto& q : aux_) CUDA_TRY(cudaStreamCreateWithFlags(&q, cudaStreamNonBlocking));
-        cudaMemPoolProps props;
-        std::memset(&props, 0, sizeof(props));
-        props.allocType = cudaMemAllocationTypePinned;
-        props.handleTypes = cudaMemHandleTypeNone;
-        props.location.type = cudaMemLocationTypeDevice;
-        props.location.id = device;
-        CUDA_TRY(cudaMemPoolCreate(&pool_, &props));
-        uint64_t keep = UINT64_MAX;
-        CUDA_TRY(cudaMemPoolSetAttribute(pool_, cudaMemPoolAttrReleaseThreshold, &keep));
+        if (int rc = acquire_server_pool(device, &pool_)) return rc;
         CUDA_TRY(cudaMalloc(&d_ctl_, 256 + 4 * sizeof(int) * kMaxInFlight));
         d_status_ = reinterpret_cast<int*>(d_ctl_ + 128);
         d_counters_ = reinterpret_cast<int*>(d_ctl_ + 256);
@@ -346,7 +404,7 @@ class Server {
         if (cfg_.hbm_budget_bytes == 0) {
             size_t fr = 0, tot = 0;
             CUDA_TRY(cudaMemGetInfo(&fr, &tot));
-            budget_ = (size_t)(0.9 * (double)fr);
+            budget_ = (size_t)(0.9 * (double)(fr + server_pool_cached()));
         } else {
             budget_ = cfg_.hbm_budget_bytes;
         }
@@ -384,7 +442,7 @@ class Server {
         if (st_) cudaStreamSynchronize(st_);
         if (d_ctl_) cudaFree(d_ctl_);
         d_ctl_ = nullptr;
-        if (pool_) cudaMemPoolDestroy(pool_);
+        if (pool_) release_server_pool();
         pool_ = nullptr;
         for (auto& q : aux_) {
             if (q) cudaStreamDestroy(q);
@@ -557,6 +615,15 @@ class Server {
         for (auto& r : active_) finish_locked(*r, kFailed, FOMO_ECUDA, error_);
         for (auto& r : retiring_) finish_locked(*r, kFailed, FOMO_ECUDA, error_);
         for (auto& r : queue_) finish_locked(*r, kFailed, FOMO_ECUDA, error_);
+        // the pool outlives the server: give back what the shots held
+        for (auto& r : active_)
+            if (r->d_block) {
+                cudaFreeAsync(r->d_block, st_);
+                r->d_block = nullptr;
+            }
+        for (auto& e : resident_) cudaFreeAsync(e.second->buoy, st_);
+        resident_.clear();
+        used_ = 0;
         active_.clear();
         retiring_.clear();
         queue_.clear();
