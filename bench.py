@@ -56,8 +56,8 @@ def parse():
                    help="offered load of the serving sample, as a multiple of the sequential plain capacity")
     p.add_argument("--no-uneven", action="store_true", help="skip the uneven-batch section")
     p.add_argument("--step-kernel", choices=["auto", "split", "fused"], default="auto",
-                   help="single-shot time-step kernels: the faster on the grid, timed on live steps (auto), "
-                        "or one of the two")
+                   help="single-shot time-step kernels: resident where the grid fits, else the faster of split and "
+                        "fused, timed on live steps (auto), or one of those two")
     p.add_argument("--segs", type=int, default=0, help="fused step: row segments per column strip (0 = auto)")
     return p.parse_args()
 
