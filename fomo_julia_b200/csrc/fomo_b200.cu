@@ -656,9 +656,16 @@ fomo::ResidentPlan shot_resident_plan(const Shot& s, const Medium& m) {
     return p;
 }
 
+int record_last(Shot& s);
+
 template <int M>
 int run_steps_resident(Shot& s, Medium& m, Wavefield& w, int n_steps, const fomo::ResidentPlan& plan) {
     auto& C = ctx();
+    const int k_end = std::min(s.nt, s.k_done + n_steps);
+    // The split and fused launches leave the last step's receivers to the
+    // launch of the next step; the resident kernel records its own steps only.
+    if (s.k_done < k_end)
+        if (int rc = record_last(s)) return rc;
     if (int rc = ensure_buoyancy(m, s.dtx, s.dtz)) return rc;
     const int blocks = plan.L.strips * plan.L.rows;
     const size_t items = (size_t)blocks * fomo::resident_mail_items(M, plan.L.h_max);
@@ -681,7 +688,6 @@ int run_steps_resident(Shot& s, Medium& m, Wavefield& w, int n_steps, const fomo
     A.status = C.d_status;
     A.mail = C.mail;
     CUDA_TRY(cudaEventRecord(C.ev0, C.stream));
-    const int k_end = std::min(s.nt, s.k_done + n_steps);
     nvtxRangePushA("fomo_b200 time loop (resident)");
     for (int k = s.k_done + 1; k <= k_end;) {
         const int n = std::min(fomo::kRMaxSteps, k_end - k + 1);
@@ -942,10 +948,10 @@ int run_steps(Shot& s, int n_steps, Profile* prof = nullptr) {
     return fail(FOMO_EINVAL, "M=%d not supported", m->M);
 }
 
-// Records the receivers of the last step done (the next velocity launch would).
 void shutdown_servers();  // server.cuh
 void destroy_server_pool();
 
+// Records the receivers of the last step done (the next velocity launch would).
 int record_last(Shot& s) {
     auto& C = ctx();
     if (s.n_rec == 0 || s.k_done < 1 || s.recorded >= s.k_done) return FOMO_OK;
