@@ -123,6 +123,7 @@ struct Shot : Object {
     int* d_rec = nullptr;           // n_rec linear offsets
     float* d_gather = nullptr;      // nt x n_rec
     int k_done = 0, recorded = 0;
+    bool no_mail = false;           // the resident kernel's mailboxes could not be allocated
     double device_ms = 0;
     int64_t launches = 0, h2d = 0, d2h = 0;
     ~Shot() override {
@@ -162,8 +163,11 @@ Context& ctx() {
 cudaError_t pool_alloc(void** p, size_t bytes) {
     auto& C = ctx();
     cudaError_t e = cudaMallocFromPoolAsync(p, bytes, C.pool, C.stream);
-    if (e == cudaErrorMemoryAllocation) {  // give the pool's cached memory back to the device, then retry once
+    if (e == cudaErrorMemoryAllocation) {  // give the cached memory back to the device, then retry once
         (void)cudaGetLastError();
+        pool_free(C.mail);  // between calls nothing reads the mailboxes
+        C.mail = nullptr;
+        C.mail_items = 0;
         cudaStreamSynchronize(C.stream);
         cudaMemPoolTrimTo(C.pool, 0);
         trim_server_pool(0);
@@ -658,8 +662,39 @@ fomo::ResidentPlan shot_resident_plan(const Shot& s, const Medium& m) {
 
 int record_last(Shot& s);
 
+// Mailboxes for `items` messages; false if the device has no room for them.
+// Messages carry the step's tag, which only grows: a mailbox is cleared when
+// it is allocated and when the tags wrap.
+bool reserve_mail(size_t items) {
+    auto& C = ctx();
+    if (items <= C.mail_items) return true;
+    pool_free(C.mail);
+    C.mail = nullptr;
+    C.mail_items = 0;
+    ulonglong2* p = nullptr;
+    if (pool_alloc((void**)&p, items * sizeof(ulonglong2)) != cudaSuccess) return false;
+    if (cudaMemsetAsync(p, 0, items * sizeof(ulonglong2), C.stream) != cudaSuccess) {
+        (void)cudaGetLastError();
+        pool_free(p);
+        return false;
+    }
+    C.mail = p;
+    C.mail_items = items;
+    return true;
+}
+
+// Launch errors that leave the context as it was: the device (or the share of
+// it that this process may use) does not hold the blocks at once.
+bool launch_refused(cudaError_t e) {
+    return e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorLaunchOutOfResources || e == cudaErrorNotSupported;
+}
+
+// Runs the steps on the resident kernel.  *refused: it could not be used for
+// the steps after s.k_done, which the caller runs on other launches (the bits
+// are the same): the mailboxes did not fit the device memory, or the
+// cooperative launch was refused.
 template <int M>
-int run_steps_resident(Shot& s, Medium& m, Wavefield& w, int n_steps, const fomo::ResidentPlan& plan) {
+int run_steps_resident(Shot& s, Medium& m, Wavefield& w, int n_steps, const fomo::ResidentPlan& plan, bool* refused) {
     auto& C = ctx();
     const int k_end = std::min(s.nt, s.k_done + n_steps);
     // The split and fused launches leave the last step's receivers to the
@@ -668,17 +703,9 @@ int run_steps_resident(Shot& s, Medium& m, Wavefield& w, int n_steps, const fomo
         if (int rc = record_last(s)) return rc;
     if (int rc = ensure_buoyancy(m, s.dtx, s.dtz)) return rc;
     const int blocks = plan.L.strips * plan.L.rows;
-    const size_t items = (size_t)blocks * fomo::resident_mail_items(M, plan.L.h_max);
-    // Messages carry the step's tag, which only grows: a mailbox is cleared
-    // when it is allocated and when the tags wrap.
-    if (items > C.mail_items) {
-        pool_free(C.mail);
-        C.mail = nullptr;
-        C.mail_items = 0;
-        const cudaError_t e = pool_alloc((void**)&C.mail, items * sizeof(ulonglong2));
-        if (e != cudaSuccess) return fail(FOMO_ENOMEM, "mailbox allocation failed: %s", cudaGetErrorString(e));
-        C.mail_items = items;
-        CUDA_TRY(cudaMemsetAsync(C.mail, 0, items * sizeof(ulonglong2), C.stream));
+    if (s.no_mail || !reserve_mail((size_t)blocks * fomo::resident_mail_items(M, plan.L.h_max))) {
+        s.no_mail = *refused = true;
+        return FOMO_OK;
     }
     fomo::ResidentArgs A;
     std::memset(&A, 0, sizeof(A));
@@ -707,7 +734,13 @@ int run_steps_resident(Shot& s, Medium& m, Wavefield& w, int n_steps, const fomo
         A.k0 = k;
         for (int q = 0; q < n; ++q) A.wav[q] = k + q <= (int)s.wavelet.size() ? s.wavelet[k + q - 1] : 0.f;
         C.mail_tag += n;
-        CUDA_TRY(fomo::resident_launch<M>(blocks, plan.smem, C.stream, P, A));
+        const cudaError_t e = fomo::resident_launch<M>(blocks, plan.smem, C.stream, P, A);
+        if (launch_refused(e)) {
+            (void)cudaGetLastError();
+            *refused = true;
+            break;
+        }
+        CUDA_TRY(e);
         s.launches += 1;
         w.cur = b;
         k += n;
@@ -803,7 +836,11 @@ int run_steps_M(Shot& s, Medium& m, Wavefield& w, int n_steps, Profile* prof) {
         const fomo::ResidentPlan res = shot_resident_plan<M>(s, m);
         if (res.ok) {
             note_step_choice(StepKey{m.nx, m.nz, M, s.nbc, m.fs, s.dtx == s.dtz});
-            return run_steps_resident<M>(s, m, w, n_steps, res);
+            const int k0 = s.k_done;
+            bool refused = false;
+            const int rc = run_steps_resident<M>(s, m, w, n_steps, res, &refused);
+            if (rc || !refused) return rc;
+            n_steps -= s.k_done - k0;
         }
     }
     const MarchPlan plan = shot_march_plan<M>(s, m);
