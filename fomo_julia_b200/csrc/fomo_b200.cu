@@ -11,6 +11,7 @@
 #include <algorithm>
 #include <cerrno>
 #include <atomic>
+#include <chrono>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
@@ -20,6 +21,7 @@
 #include <utility>
 #include <mutex>
 #include <string>
+#include <thread>
 #include <unordered_map>
 #include <vector>
 
@@ -145,6 +147,7 @@ struct Context {
     ulonglong2* mail = nullptr;  // mailboxes of the resident kernel, and their number of messages
     size_t mail_items = 0;
     uint32_t mail_tag = 1;       // tag of the next resident step (0: never sent)
+    std::chrono::steady_clock::time_point resident_after;  // earliest next resident launch beside served shots
     unsigned char* pinned = nullptr;  // host staging of small read-backs (kPinnedBytes), the status word first
     uint64_t next = 1;
     std::unordered_map<uint64_t, std::unique_ptr<Object>> objs;
@@ -829,20 +832,9 @@ void note_step_choice(const StepKey& k) {
     if (g_step_choice.emplace(k, 0).second) save_step_choice(k, 0);
 }
 
+// Steps on the split launches or the fused step, as `mode` (FOMO_STEP_*) says.
 template <int M>
-int run_steps_M(Shot& s, Medium& m, Wavefield& w, int n_steps, Profile* prof) {
-    const int mode = g_step_mode.load();
-    if (mode == FOMO_STEP_AUTO && !prof) {
-        const fomo::ResidentPlan res = shot_resident_plan<M>(s, m);
-        if (res.ok) {
-            note_step_choice(StepKey{m.nx, m.nz, M, s.nbc, m.fs, s.dtx == s.dtz});
-            const int k0 = s.k_done;
-            bool refused = false;
-            const int rc = run_steps_resident<M>(s, m, w, n_steps, res, &refused);
-            if (rc || !refused) return rc;
-            n_steps -= s.k_done - k0;
-        }
-    }
+int run_steps_launches(Shot& s, Medium& m, Wavefield& w, int n_steps, Profile* prof, int mode) {
     const MarchPlan plan = shot_march_plan<M>(s, m);
     if (!plan.ok) {
         if (mode == FOMO_STEP_FUSED) return fail(FOMO_EINVAL, "the fused step does not support this shot: %s", plan.why);
@@ -878,6 +870,48 @@ int run_steps_M(Shot& s, Medium& m, Wavefield& w, int n_steps, Profile* prof) {
         if (choice == 1) return run_steps_march<M>(s, m, w, n_steps, prof, plan);
     }
     return run_steps_split<M>(s, m, w, n_steps, prof);
+}
+
+// Shots submitted to servers and not finished yet.
+std::atomic<int> g_served{0};
+
+// A resident launch holds the whole device, and a server's launches get
+// nothing done meanwhile.  Beside served shots a single shot therefore takes a
+// quarter of the device's time: launches of kServedSteps steps, each followed
+// by kServedPause times its own duration for the server.  Measured on one B200,
+// single shots (508 x 308, 500 steps) one after another beside 16 served shots
+// on 2108 x 908 (135 ms without them): launches of 256 steps without pauses
+// 7.4 ms a shot, the server 1585 ms; split launches 139 and 138; this 33 and
+// 166.  Beside 24 served shots on 508 x 308 (103 ms): 7.2 and 1278, 36 and 116,
+// 34 and 125.
+using HostClock = std::chrono::steady_clock;
+constexpr int kServedSteps = 32, kServedPause = 3;
+constexpr auto kServedPauseMax = std::chrono::milliseconds(100);  // a launch that itself waited long
+
+template <int M>
+int run_steps_M(Shot& s, Medium& m, Wavefield& w, int n_steps, Profile* prof) {
+    auto& C = ctx();
+    const int mode = g_step_mode.load();
+    if (mode == FOMO_STEP_AUTO && !prof) {
+        const fomo::ResidentPlan res = shot_resident_plan<M>(s, m);
+        if (res.ok) {
+            note_step_choice(StepKey{m.nx, m.nz, M, s.nbc, m.fs, s.dtx == s.dtz});
+            bool refused = false;
+            do {
+                while (g_served.load() > 0 && HostClock::now() < C.resident_after)
+                    std::this_thread::sleep_for(std::chrono::microseconds(100));
+                const bool served = g_served.load() > 0;
+                const int n = served ? std::min(n_steps, kServedSteps) : n_steps, k0 = s.k_done;
+                const auto t0 = HostClock::now();
+                if (int rc = run_steps_resident<M>(s, m, w, n, res, &refused)) return rc;
+                const auto t1 = HostClock::now();
+                if (served) C.resident_after = t1 + std::min<HostClock::duration>(kServedPause * (t1 - t0), kServedPauseMax);
+                n_steps -= refused ? s.k_done - k0 : n;
+            } while (!refused && n_steps > 0 && s.k_done < s.nt);
+            if (!refused) return FOMO_OK;
+        }
+    }
+    return run_steps_launches<M>(s, m, w, n_steps, prof, mode);
 }
 
 // The split launches: velocity tiles, velocity band pass, stress tiles,

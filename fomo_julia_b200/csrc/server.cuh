@@ -602,6 +602,7 @@ class Server {
         if (r.med) {
             r.med->users.fetch_sub(1);
             r.med = nullptr;
+            g_served.fetch_sub(1);
         }
         cv_done_.notify_all();
     }
@@ -1502,9 +1503,11 @@ int fomo_b200_server_submit(uint64_t server, uint64_t medium, const FomoHabc* ha
         if (!m) return fail(FOMO_EINVAL, "unknown medium handle %llu", (unsigned long long)medium);
         if (int rc = make_request(m, habc, shot, gather_out, &r)) return rc;
         m->users.fetch_add(1);
+        g_served.fetch_add(1);
     }
     if (int rc = s->submit(r, ticket)) {
         r->med->users.fetch_sub(1);
+        g_served.fetch_sub(1);
         return rc;
     }
     return FOMO_OK;

@@ -114,6 +114,7 @@ cudaError_t cudaLaunchCooperativeKernel(const void* f, dim3, dim3, void**, size_
     std::lock_guard<std::recursive_mutex> lk(mu);
     if (after >= 0 && counts["cooperative"] >= after) return note(cudaErrorCooperativeLaunchTooLarge);
     counts["cooperative"] += 1;
+    usleep((useconds_t)setting("launch_us"));
     return launch(f);
 }
 

@@ -108,3 +108,40 @@ s.advance(500)                                            # allocated again
 assert s.k.value == 600 and get("launches:" + SPLIT) == 0
 s.finish()
 """)
+
+
+def test_single_shots_beside_served_ones_share_the_device(host_run):
+    host_run("""
+c = case()
+s = OpenShot(c, b)
+H = F.init_habc(s.med.nx, s.med.nz, c.nbc, c.dt, c.dx, c.dz, c.v_ref, b)
+a, par = F.get_fd_coefficients(8), F.sim_params(c.dt, c.nt, c.dx, c.dz, 8)
+src, rec = F.Source(60, 30, F.ricker_wavelet(c.f0, c.dt, c.nt)), F.setup_receivers(c.rec_x, c.rec_z, s.med)
+with F.ShotServer() as srv:
+    put("hold", 1)
+    t = srv.submit(s.med, H, a, src, rec, par)
+    bad = F.Source(10 ** 6, 30, src.wavelet)
+    try:
+        srv.submit(s.med, H, a, bad, rec, par)            # refused: not in flight
+    except F._lib.FomoError:
+        pass
+    t0 = time.time()
+    s.advance(40)                                         # the served shot is in flight: launches of 32 steps
+    assert get("launches:resident_kernel") == 2
+    put("launch_us", 20000)
+    s.advance(70)                                         # three launches, the first two with pauses of three times their time
+    assert get("launches:resident_kernel") == 5 and time.time() - t0 > 2 * 0.06 + 3 * 0.02
+    put("launch_us", 0)
+    put("hold", 0)
+    srv.wait(t, timeout=60)
+    t0 = time.time()
+    s.advance(490)                                        # alone again: at once, 256 steps a launch
+    assert s.k.value == 600 and get("launches:resident_kernel") == 7 and time.time() - t0 < 0.05
+    put("hold", 1)
+    more = [srv.submit(s.med, H, a, src, rec, par) for _ in range(3)]
+    put("hold", 0)
+    srv.wait_all(more, timeout=60)
+    s2 = OpenShot(c, b)
+    s2.advance(600)
+    assert get("launches:resident_kernel") == 10 and get("launches:" + SPLIT) == 0
+""")
