@@ -653,28 +653,36 @@ class Server {
             *rc = fail(FOMO_ENOMEM, "buoyancy allocation of %zu bytes failed", R->bytes);
             return nullptr;
         }
-        float* b0 = R->buoy;
-        float* b2 = R->buoy + plane;
-        float* b1 = R->iso ? b0 : R->buoy + 2 * plane;
-        float* b3 = R->iso ? b2 : R->buoy + 3 * plane;
-        fomo::buoyancy_kernel<<<4 * sm_count(), 256, 0, st_>>>(m.arr(0), m.arr(1), r.dtx, r.dtz, plane, b0, b1, b2, b3);
-        if (cudaGetLastError() != cudaSuccess) {
-            *rc = fail(FOMO_ECUDA, "buoyancy kernel launch failed");
+        if ((*rc = fill_resident(r, *R))) {
+            cudaFreeAsync(R->buoy, st_);
             return nullptr;
         }
-        count_launches(1);
-        R->b[0] = b0;
-        R->b[1] = b1;
-        R->b[2] = b2;
-        R->b[3] = b3;
-        for (int q = 0; q < 4; ++q)
-            if ((*rc = encode_map(&R->bmap[q], R->b[q], m.nx, m.nz, m.pitch, fomo::kTX, fomo::kTZ))) return nullptr;
-        for (int q = 0; q < 3; ++q)
-            if ((*rc = encode_map(&R->mod[q], m.arr(2 + q), m.nx, m.nz, m.pitch, fomo::kTX, fomo::kTZ))) return nullptr;
         used_ += R->bytes;
         Resident* p = R.get();
         resident_.emplace(key, std::move(R));
         return p;
+    }
+
+    // Computes a medium's buoyancy arrays and encodes its tile boxes.
+    int fill_resident(Request& r, Resident& R) {
+        const Medium& m = *r.med;
+        const size_t plane = (size_t)m.pitch * m.nz;
+        float* b0 = R.buoy;
+        float* b2 = R.buoy + plane;
+        float* b1 = R.iso ? b0 : R.buoy + 2 * plane;
+        float* b3 = R.iso ? b2 : R.buoy + 3 * plane;
+        fomo::buoyancy_kernel<<<4 * sm_count(), 256, 0, st_>>>(m.arr(0), m.arr(1), r.dtx, r.dtz, plane, b0, b1, b2, b3);
+        if (cudaGetLastError() != cudaSuccess) return fail(FOMO_ECUDA, "buoyancy kernel launch failed");
+        count_launches(1);
+        R.b[0] = b0;
+        R.b[1] = b1;
+        R.b[2] = b2;
+        R.b[3] = b3;
+        for (int q = 0; q < 4; ++q)
+            if (int rc = encode_map(&R.bmap[q], R.b[q], m.nx, m.nz, m.pitch, fomo::kTX, fomo::kTZ)) return rc;
+        for (int q = 0; q < 3; ++q)
+            if (int rc = encode_map(&R.mod[q], m.arr(2 + q), m.nx, m.nz, m.pitch, fomo::kTX, fomo::kTZ)) return rc;
+        return FOMO_OK;
     }
 
     template <int M>

@@ -31,7 +31,7 @@ std::map<std::string, long> launches;
 std::map<void*, Block> blocks;
 std::map<Pool*, int> pools;
 std::map<std::string, long> settings, counts;
-cudaError_t last = cudaSuccess;
+thread_local cudaError_t last = cudaSuccess;
 
 long setting(const char* k, long dflt = 0) {
     std::lock_guard<std::recursive_mutex> lk(mu);
@@ -54,7 +54,7 @@ cudaError_t launch(const void* f) {
     launches[kernels[f]] += 1;
     return cudaSuccess;
 }
-CUresult encode(...) { return CUDA_SUCCESS; }
+CUresult encode(...) { return setting("fail_encode") ? CUDA_ERROR_INVALID_VALUE : CUDA_SUCCESS; }
 // Waits while fake_set("hold", 1): work enqueued on a stream that does not finish yet.
 void held() {
     while (setting("hold")) usleep(200);
@@ -202,8 +202,10 @@ cudaError_t cudaMemPoolTrimTo(cudaMemPool_t p, size_t keep) {
     if (q->reserved > keep) q->reserved = keep > q->used ? keep : q->used;
     return cudaSuccess;
 }
-cudaError_t cudaMallocFromPoolAsync(void** ptr, size_t n, cudaMemPool_t p, cudaStream_t) {
+// fake_set("scale", k): a block counts k times its size in its pool
+cudaError_t cudaMallocFromPoolAsync(void** ptr, size_t bytes, cudaMemPool_t p, cudaStream_t) {
     const long lo = setting("fail_alloc_min", -1), hi = setting("fail_alloc_max", -1);
+    const size_t n = bytes * (size_t)setting("scale", 1);
     std::lock_guard<std::recursive_mutex> lk(mu);
     Pool* q = live_pool(p);
     if (!q) return note(cudaErrorInvalidValue);
@@ -215,7 +217,7 @@ cudaError_t cudaMallocFromPoolAsync(void** ptr, size_t n, cudaMemPool_t p, cudaS
     }
     q->used += n;
     q->reserved += grow;
-    blocks[*ptr = std::calloc(n ? n : 1, 1)] = Block{q, n};
+    blocks[*ptr = std::calloc(bytes ? bytes : 1, 1)] = Block{q, n};
     return cudaSuccess;
 }
 cudaError_t cudaFreeAsync(void* p, cudaStream_t) {

@@ -145,3 +145,41 @@ with F.ShotServer() as srv:
     s2.advance(600)
     assert get("launches:resident_kernel") == 10 and get("launches:" + SPLIT) == 0
 """)
+
+
+SERVED = """
+c = case(nt=40, n_rec=5)
+med = F.init_medium(c.vp, c.vs, c.rho, c.dx, c.dz, c.nbc, 8, b)
+H = F.init_habc(med.nx, med.nz, c.nbc, c.dt, c.dx, c.dz, c.v_ref, b)
+a, par = F.get_fd_coefficients(8), F.sim_params(c.dt, c.nt, c.dx, c.dz, 8)
+src, rec = F.Source(60, 30, F.ricker_wavelet(c.f0, c.dt, c.nt)), F.setup_receivers(c.rec_x, c.rec_z, med)
+submit = lambda srv, p=par, r=rec: srv.submit(med, H, a, src, r, p)
+def wait(srv, t):
+    try:
+        srv.wait(t, timeout=60)
+        return ""
+    except F._lib.FomoError as e:
+        return str(e)
+med.upload()
+"""
+
+
+def test_failed_server_leaves_no_device_memory(host_run):
+    host_run(SERVED + """
+before = get("live_bytes")
+for failing in ("fail_encode", "fail_alloc_min"):
+    with F.ShotServer() as srv:
+        t0 = submit(srv)
+        assert wait(srv, t0) == ""
+        put("fail_alloc_max", 1 << 40); put(failing, 1)
+        assert "failed" in wait(srv, submit(srv))
+        put("fail_encode", 0); put("fail_alloc_min", -1)
+        try:
+            submit(srv)
+            raise AssertionError("a failed server took a shot")
+        except F._lib.FomoError as e:
+            assert "server failed" in str(e)
+    assert get("live_bytes") == before, failing
+with F.ShotServer() as srv:
+    assert wait(srv, submit(srv)) == ""
+""")
