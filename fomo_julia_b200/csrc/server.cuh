@@ -326,47 +326,57 @@ cudaError_t launch_batch(bool vel, const LaunchSet& S, cudaStream_t st, bool aft
 // mapping a batch's memory anew took 7-20 ms of it, many times that on some
 // hosts).  What is freed stays mapped while a server lives; once the last one
 // is gone kServerPoolKeep bytes stay, until the library needs the memory or
-// shuts down.  The pool orders reuse across the servers' streams itself.
+// shuts down.  The pool orders reuse across the servers' streams itself, and
+// lives as long as a server uses it.
 constexpr size_t kServerPoolKeep = 2ull << 30;
 struct ServerPool {
-    std::mutex mu;
     cudaMemPool_t pool = nullptr;
     int servers = 0;
+    ~ServerPool() {
+        if (pool) cudaMemPoolDestroy(pool);
+    }
 };
-ServerPool& server_pool() {
-    static ServerPool p;
-    return p;
+struct ServerPoolSlot {
+    std::mutex mu;  // guards the pool's servers too
+    std::shared_ptr<ServerPool> pool;
+};
+ServerPoolSlot& server_pool() {
+    static ServerPoolSlot& s = *new ServerPoolSlot;  // never destroyed: no CUDA call at exit
+    return s;
 }
 
-int acquire_server_pool(int device, cudaMemPool_t* out) {
+int acquire_server_pool(int device, std::shared_ptr<ServerPool>* out) {
     auto& S = server_pool();
     std::lock_guard<std::mutex> lk(S.mu);
     if (!S.pool) {
+        auto p = std::make_shared<ServerPool>();
         cudaMemPoolProps props;
         std::memset(&props, 0, sizeof(props));
         props.allocType = cudaMemAllocationTypePinned;
         props.handleTypes = cudaMemHandleTypeNone;
         props.location.type = cudaMemLocationTypeDevice;
         props.location.id = device;
-        CUDA_TRY(cudaMemPoolCreate(&S.pool, &props));
+        CUDA_TRY(cudaMemPoolCreate(&p->pool, &props));
         uint64_t keep = UINT64_MAX;
-        CUDA_TRY(cudaMemPoolSetAttribute(S.pool, cudaMemPoolAttrReleaseThreshold, &keep));
+        CUDA_TRY(cudaMemPoolSetAttribute(p->pool, cudaMemPoolAttrReleaseThreshold, &keep));
+        S.pool = p;
     }
-    S.servers += 1;
+    S.pool->servers += 1;
     *out = S.pool;
     return FOMO_OK;
 }
 
-void release_server_pool() {
+void release_server_pool(std::shared_ptr<ServerPool>& p) {
     auto& S = server_pool();
     std::lock_guard<std::mutex> lk(S.mu);
-    if (--S.servers == 0) cudaMemPoolTrimTo(S.pool, kServerPoolKeep);
+    if (--p->servers == 0 && S.pool == p) cudaMemPoolTrimTo(p->pool, kServerPoolKeep);
+    p.reset();
 }
 
 void trim_server_pool(size_t keep) {
     auto& S = server_pool();
     std::lock_guard<std::mutex> lk(S.mu);
-    if (S.pool) cudaMemPoolTrimTo(S.pool, keep);
+    if (S.pool) cudaMemPoolTrimTo(S.pool->pool, keep);
 }
 
 // Mapped and unused bytes of the pool: a new server can have them too.
@@ -374,17 +384,17 @@ size_t server_pool_cached() {
     auto& S = server_pool();
     std::lock_guard<std::mutex> lk(S.mu);
     uint64_t reserved = 0, used = 0;
-    if (!S.pool || cudaMemPoolGetAttribute(S.pool, cudaMemPoolAttrReservedMemCurrent, &reserved) != cudaSuccess ||
-        cudaMemPoolGetAttribute(S.pool, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess)
+    if (!S.pool || cudaMemPoolGetAttribute(S.pool->pool, cudaMemPoolAttrReservedMemCurrent, &reserved) != cudaSuccess ||
+        cudaMemPoolGetAttribute(S.pool->pool, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess)
         return 0;
     return reserved > used ? (size_t)(reserved - used) : 0;
 }
 
-void destroy_server_pool() {  // no server is left
+// The library shuts down: the pool goes with its last server.
+void destroy_server_pool() {
     auto& S = server_pool();
     std::lock_guard<std::mutex> lk(S.mu);
-    if (S.pool) cudaMemPoolDestroy(S.pool);
-    S.pool = nullptr;
+    S.pool.reset();
 }
 
 class Server {
@@ -442,8 +452,7 @@ class Server {
         if (st_) cudaStreamSynchronize(st_);
         if (d_ctl_) cudaFree(d_ctl_);
         d_ctl_ = nullptr;
-        if (pool_) release_server_pool();
-        pool_ = nullptr;
+        if (pool_) release_server_pool(pool_);
         for (auto& q : aux_) {
             if (q) cudaStreamDestroy(q);
             q = nullptr;
@@ -540,7 +549,7 @@ class Server {
     size_t budget_ = 0;
     cudaStream_t st_ = nullptr;
     cudaStream_t aux_[kChains - 1] = {};  // the further chains' streams, idle between chunks
-    cudaMemPool_t pool_ = nullptr;
+    std::shared_ptr<ServerPool> pool_;
     unsigned char* d_ctl_ = nullptr;
     int* d_counters_ = nullptr;   // per launch set: velocity and stress batch step
     int* d_status_ = nullptr;
@@ -649,7 +658,7 @@ class Server {
         R->iso = r.dtx == r.dtz ? 1 : 0;
         const size_t plane = (size_t)m.pitch * m.nz;
         R->bytes = (R->iso ? 2 : 4) * plane * sizeof(float);
-        if (cudaMallocFromPoolAsync(reinterpret_cast<void**>(&R->buoy), R->bytes, pool_, st_) != cudaSuccess) {
+        if (cudaMallocFromPoolAsync(reinterpret_cast<void**>(&R->buoy), R->bytes, pool_->pool, st_) != cudaSuccess) {
             *rc = fail(FOMO_ENOMEM, "buoyancy allocation of %zu bytes failed", R->bytes);
             return nullptr;
         }
@@ -747,7 +756,7 @@ class Server {
         r.wav_off = r.cells_off + align_up(r.cells.size() * 4, 256);
         r.gather_off = r.wav_off + align_up(std::max<size_t>(r.wavelet.size(), 1) * 4, 256);
         const size_t total = r.gather_off + align_up((size_t)r.nt * r.n_rec * 4, 256);
-        if (cudaMallocFromPoolAsync(reinterpret_cast<void**>(&r.d_block), total, pool_, st_) != cudaSuccess)
+        if (cudaMallocFromPoolAsync(reinterpret_cast<void**>(&r.d_block), total, pool_->pool, st_) != cudaSuccess)
             return fail(FOMO_ENOMEM, "shot allocation of %zu bytes failed", total);
         r.bytes = total;
         used_ += total;

@@ -234,10 +234,13 @@ cudaError_t cudaMalloc(void** p, size_t n) {
     blocks[*p = std::calloc(n, 1)] = Block{nullptr, n};
     return cudaSuccess;
 }
-// fake_set("hold_free", 1): waits, as cudaFree waits for the device
+// fake_set("hold_free", 1): waits, as cudaFree waits for the device ("in_free" counts the calls that did)
 cudaError_t cudaFree(void* p) {
     if (setting("hold_free")) {
-        fake_set("in_free", 1);
+        {
+            std::lock_guard<std::recursive_mutex> lk(mu);
+            counts["in_free"] += 1;
+        }
         while (setting("hold_free")) usleep(200);
     }
     return cudaFreeAsync(p, nullptr);

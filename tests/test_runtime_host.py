@@ -45,7 +45,7 @@ def host_run(tmp_path_factory):
         e = {k: v for k, v in os.environ.items() if not k.startswith("FOMO_B200_")}
         e.update(LD_PRELOAD=str(so), PYTHONDONTWRITEBYTECODE="1", **env)
         r = subprocess.run([sys.executable, "-c", PRELUDE.format(here=HERE) + script], capture_output=True, text=True,
-                           env=e, timeout=120)
+                           env=e, timeout=60)
         assert r.returncode == 0, r.stdout + r.stderr
         return r.stdout
 
@@ -180,6 +180,31 @@ for failing in ("fail_encode", "fail_alloc_min"):
         except F._lib.FomoError as e:
             assert "server failed" in str(e)
     assert get("live_bytes") == before, failing
+with F.ShotServer() as srv:
+    assert wait(srv, submit(srv)) == ""
+""")
+
+
+def test_library_shutdown_while_a_server_closes(host_run):
+    host_run(SERVED + """
+srv = F.ShotServer()
+assert wait(srv, submit(srv)) == ""
+put("hold_free", 1)
+t = threading.Thread(target=srv.close)
+t.start()
+while not get("in_free"):                                 # the server has left the table of servers
+    time.sleep(0.001)
+down = threading.Thread(target=lambda: F._lib.call("fomo_b200_shutdown"))
+down.start()
+time.sleep(0.2)
+put("hold_free", 0)
+t.join(); down.join()
+assert get("bad_pool_calls") == 0 and get("pools") == 0
+F._lib._inited_device = None
+F._lib.ensure_init(0)                                     # and the library starts again
+W = F.Wavefield(60, 40, b)
+med = F.init_medium(c.vp, c.vs, c.rho, c.dx, c.dz, c.nbc, 8, b)
+med.upload()
 with F.ShotServer() as srv:
     assert wait(srv, submit(srv)) == ""
 """)
