@@ -70,7 +70,7 @@ struct Buffer : Object {
 // and no device-wide synchronisation (cudaFree has both).
 cudaError_t pool_alloc(void** p, size_t bytes);
 void pool_free(void* p);
-void trim_server_pool(size_t keep);  // server.cuh
+void trim_server_pool();  // server.cuh
 
 // Row pitch in floats: rows start on 128-byte boundaries.
 inline int pitch_of(int nx) { return (nx + 31) / 32 * 32; }
@@ -173,7 +173,7 @@ cudaError_t pool_alloc(void** p, size_t bytes) {
         C.mail_items = 0;
         cudaStreamSynchronize(C.stream);
         cudaMemPoolTrimTo(C.pool, 0);
-        trim_server_pool(0);
+        trim_server_pool();
         e = cudaMallocFromPoolAsync(p, bytes, C.pool, C.stream);
     }
     if (e != cudaSuccess) {

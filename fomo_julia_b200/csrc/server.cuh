@@ -324,16 +324,21 @@ cudaError_t launch_batch(bool vel, const LaunchSet& S, cudaStream_t st, bool aft
 // Device memory of the servers' shots: one stream-ordered pool for all of
 // them, kept between servers (fomo_b200_run_batch makes one for each call, and
 // mapping a batch's memory anew took 7-20 ms of it, many times that on some
-// hosts).  What is freed stays mapped while a server lives; once the last one
-// is gone kServerPoolKeep bytes stay, until the library needs the memory or
-// shuts down.  The pool orders reuse across the servers' streams itself, and
-// lives as long as a server uses it.
+// hosts).  A server keeps what it has mapped, the most it held at once, while
+// it lives; beyond that kServerPoolKeep bytes stay when a server is gone, until
+// the library needs the memory or shuts down.  The pool orders reuse across
+// the servers' streams itself, and lives as long as a server uses it.
 constexpr size_t kServerPoolKeep = 2ull << 30;
 struct ServerPool {
     cudaMemPool_t pool = nullptr;
-    int servers = 0;
+    std::vector<const std::atomic<size_t>*> peaks;  // of each server on it: the most bytes it held at once
     ~ServerPool() {
         if (pool) cudaMemPoolDestroy(pool);
+    }
+    size_t claimed() const {
+        size_t n = 0;
+        for (auto* p : peaks) n += p->load();
+        return n;
     }
 };
 struct ServerPoolSlot {
@@ -345,7 +350,9 @@ ServerPoolSlot& server_pool() {
     return s;
 }
 
-int acquire_server_pool(int device, std::shared_ptr<ServerPool>* out) {
+// The pool for a server; *available: the free device memory and what the pool
+// has mapped beyond the other servers' share.
+int acquire_server_pool(int device, const std::atomic<size_t>* peak, std::shared_ptr<ServerPool>* out, size_t* available) {
     auto& S = server_pool();
     std::lock_guard<std::mutex> lk(S.mu);
     if (!S.pool) {
@@ -361,33 +368,31 @@ int acquire_server_pool(int device, std::shared_ptr<ServerPool>* out) {
         CUDA_TRY(cudaMemPoolSetAttribute(p->pool, cudaMemPoolAttrReleaseThreshold, &keep));
         S.pool = p;
     }
-    S.pool->servers += 1;
+    size_t fr = 0, tot = 0;
+    uint64_t reserved = 0, used = 0;
+    CUDA_TRY(cudaMemGetInfo(&fr, &tot));
+    CUDA_TRY(cudaMemPoolGetAttribute(S.pool->pool, cudaMemPoolAttrReservedMemCurrent, &reserved));
+    CUDA_TRY(cudaMemPoolGetAttribute(S.pool->pool, cudaMemPoolAttrUsedMemCurrent, &used));
+    const uint64_t taken = std::max<uint64_t>(used, S.pool->claimed());
+    *available = fr + (reserved > taken ? (size_t)(reserved - taken) : 0);
+    S.pool->peaks.push_back(peak);
     *out = S.pool;
     return FOMO_OK;
 }
 
-void release_server_pool(std::shared_ptr<ServerPool>& p) {
+void release_server_pool(std::shared_ptr<ServerPool>& p, const std::atomic<size_t>* peak) {
     auto& S = server_pool();
     std::lock_guard<std::mutex> lk(S.mu);
-    if (--p->servers == 0 && S.pool == p) cudaMemPoolTrimTo(p->pool, kServerPoolKeep);
+    p->peaks.erase(std::find(p->peaks.begin(), p->peaks.end(), peak));
+    if (S.pool == p) cudaMemPoolTrimTo(p->pool, p->claimed() + kServerPoolKeep);
     p.reset();
 }
 
-void trim_server_pool(size_t keep) {
+// The library needs device memory: the pool gives back all but its servers' share.
+void trim_server_pool() {
     auto& S = server_pool();
     std::lock_guard<std::mutex> lk(S.mu);
-    if (S.pool) cudaMemPoolTrimTo(S.pool->pool, keep);
-}
-
-// Mapped and unused bytes of the pool: a new server can have them too.
-size_t server_pool_cached() {
-    auto& S = server_pool();
-    std::lock_guard<std::mutex> lk(S.mu);
-    uint64_t reserved = 0, used = 0;
-    if (!S.pool || cudaMemPoolGetAttribute(S.pool->pool, cudaMemPoolAttrReservedMemCurrent, &reserved) != cudaSuccess ||
-        cudaMemPoolGetAttribute(S.pool->pool, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess)
-        return 0;
-    return reserved > used ? (size_t)(reserved - used) : 0;
+    if (S.pool) cudaMemPoolTrimTo(S.pool->pool, S.pool->claimed());
 }
 
 // The library shuts down: the pool goes with its last server.
@@ -406,18 +411,13 @@ class Server {
         CUDA_TRY(cudaSetDevice(device));
         CUDA_TRY(cudaStreamCreateWithFlags(&st_, cudaStreamNonBlocking));
         for (auto& q : aux_) CUDA_TRY(cudaStreamCreateWithFlags(&q, cudaStreamNonBlocking));
-        if (int rc = acquire_server_pool(device, &pool_)) return rc;
+        size_t available = 0;
+        if (int rc = acquire_server_pool(device, &peak_, &pool_, &available)) return rc;
         CUDA_TRY(cudaMalloc(&d_ctl_, 256 + 4 * sizeof(int) * kMaxInFlight));
         d_status_ = reinterpret_cast<int*>(d_ctl_ + 128);
         d_counters_ = reinterpret_cast<int*>(d_ctl_ + 256);
         CUDA_TRY(cudaMemset(d_status_, 0, sizeof(int)));
-        if (cfg_.hbm_budget_bytes == 0) {
-            size_t fr = 0, tot = 0;
-            CUDA_TRY(cudaMemGetInfo(&fr, &tot));
-            budget_ = (size_t)(0.9 * (double)(fr + server_pool_cached()));
-        } else {
-            budget_ = cfg_.hbm_budget_bytes;
-        }
+        budget_ = cfg_.hbm_budget_bytes ? cfg_.hbm_budget_bytes : (size_t)(0.9 * (double)available);
         {
             std::lock_guard<std::mutex> lk(g_tune_mu);
             load_tune_cache();
@@ -452,7 +452,7 @@ class Server {
         if (st_) cudaStreamSynchronize(st_);
         if (d_ctl_) cudaFree(d_ctl_);
         d_ctl_ = nullptr;
-        if (pool_) release_server_pool(pool_);
+        if (pool_) release_server_pool(pool_, &peak_);
         for (auto& q : aux_) {
             if (q) cudaStreamDestroy(q);
             q = nullptr;
@@ -550,6 +550,7 @@ class Server {
     cudaStream_t st_ = nullptr;
     cudaStream_t aux_[kChains - 1] = {};  // the further chains' streams, idle between chunks
     std::shared_ptr<ServerPool> pool_;
+    std::atomic<size_t> peak_{0};         // the most device bytes held at once
     unsigned char* d_ctl_ = nullptr;
     int* d_counters_ = nullptr;   // per launch set: velocity and stress batch step
     int* d_status_ = nullptr;
@@ -634,6 +635,7 @@ class Server {
         for (auto& e : resident_) cudaFreeAsync(e.second->buoy, st_);
         resident_.clear();
         used_ = 0;
+        peak_.store(0);
         active_.clear();
         retiring_.clear();
         queue_.clear();
@@ -666,7 +668,7 @@ class Server {
             cudaFreeAsync(R->buoy, st_);
             return nullptr;
         }
-        used_ += R->bytes;
+        hold(R->bytes);
         Resident* p = R.get();
         resident_.emplace(key, std::move(R));
         return p;
@@ -692,6 +694,12 @@ class Server {
         for (int q = 0; q < 3; ++q)
             if (int rc = encode_map(&R.mod[q], m.arr(2 + q), m.nx, m.nz, m.pitch, fomo::kTX, fomo::kTZ)) return rc;
         return FOMO_OK;
+    }
+
+    // Counts device bytes as held by the server.
+    void hold(size_t bytes) {
+        used_ += bytes;
+        if (used_ > peak_.load()) peak_.store(used_);
     }
 
     template <int M>
@@ -759,7 +767,7 @@ class Server {
         if (cudaMallocFromPoolAsync(reinterpret_cast<void**>(&r.d_block), total, pool_->pool, st_) != cudaSuccess)
             return fail(FOMO_ENOMEM, "shot allocation of %zu bytes failed", total);
         r.bytes = total;
-        used_ += total;
+        hold(total);
         unsigned char* base = r.d_block;
         CUDA_TRY(cudaMemsetAsync(base, 0, 10 * plane, st_));
         std::memcpy(stage, r.tabs.data(), r.tabs.size() * 4);

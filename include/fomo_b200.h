@@ -352,7 +352,9 @@ int fomo_b200_run_batch(uint64_t medium, const FomoHabc* habc, const FomoShot* s
  * on the device whatever their media, orders and nt, and each result equals
  * fomo_b200_run_shot's bit for bit. */
 typedef struct {
-    uint64_t hbm_budget_bytes;  /* device bytes for shots; 0 = 90% of free memory   */
+    uint64_t hbm_budget_bytes;  /* device bytes for shots; 0 = 90% of the device's  */
+                                /* free memory, counting what earlier servers left  */
+                                /* mapped but not what running servers hold         */
     int32_t max_shots;          /* shots on the device at once; 0 = budget only      */
     int32_t steps_per_launch;   /* K; 0 = 8 (or the FOMO_B200_TUNE_CACHE file's),   */
                                 /* 1 = one launch per kernel per step, no graphs     */

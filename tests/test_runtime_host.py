@@ -208,3 +208,63 @@ med.upload()
 with F.ShotServer() as srv:
     assert wait(srv, submit(srv)) == ""
 """)
+
+
+def test_servers_keep_their_share_of_the_pool(host_run):
+    """What an idle server mapped is neither in another's budget nor taken by the library."""
+    host_run(SERVED + """
+import re
+def budget(srv):
+    long = F.sim_params(c.dt, 1 << 26, c.dx, c.dz, 8)     # a gather of 1.3 GB
+    try:
+        submit(srv, long)
+        raise AssertionError("took a shot larger than the device")
+    except F._lib.FomoError as e:
+        return int(re.search(r"HBM budget of (\\d+)", str(e)).group(1))
+cap = get("reserved") + (200 << 20)
+put("capacity", cap)
+A = F.ShotServer(hbm_budget_bytes=100 << 20)
+put("hold", 1)
+ts = [submit(A) for _ in range(40)]
+put("hold", 0)
+assert all(wait(A, t) == "" for t in ts)
+share = A.stats()["peak_bytes"]
+free = (200 << 20) - share
+assert share > 10 << 20
+with F.ShotServer() as B:                                 # free memory only
+    assert abs(budget(B) - 0.9 * free) < 1 << 20, (budget(B), share)
+try:                                                      # the library may not have it either
+    F.Wavefield(2048, (free + share // 2) // (10 * 4 * 2048), b)
+    raise AssertionError("the library took a live server's memory")
+except F._lib.FomoError as e:
+    assert "FOMO_ENOMEM" in str(e)
+W = F.Wavefield(2048, int(free * 0.95) // (10 * 4 * 2048), b)
+put("hold", 1)
+ts = [submit(A) for _ in range(40)]
+put("hold", 0)
+assert all(wait(A, t) == "" for t in ts)                  # its burst still fits
+W.release()
+A.close()
+with F.ShotServer() as B:                                 # what a closed server mapped counts as free
+    assert abs(budget(B) - 0.9 * (cap - get("reserved") + share)) < 1 << 20
+""")
+
+
+def test_memory_of_a_closed_server_is_bounded_beside_a_live_one(host_run):
+    host_run(SERVED + """
+A = F.ShotServer()
+assert wait(A, submit(A)) == ""
+share = A.stats()["peak_bytes"]
+base = get("reserved")
+put("scale", 1000)                                        # 0.9 GB a shot
+with F.ShotServer() as B:
+    put("hold", 1)
+    ts = [submit(B) for _ in range(8)]
+    put("hold", 0)
+    assert all(wait(B, t) == "" for t in ts)
+    assert get("reserved") - base > 4 << 30
+put("scale", 1)
+assert get("reserved") - base <= share + (2 << 30)
+assert wait(A, submit(A)) == ""
+A.close()
+""")
