@@ -877,15 +877,15 @@ std::atomic<int> g_served{0};
 
 // A resident launch holds the whole device, and a server's launches get
 // nothing done meanwhile.  Beside served shots a single shot therefore takes a
-// quarter of the device's time: launches of kServedSteps steps, each followed
-// by kServedPause times its own duration for the server.  Measured on one B200,
-// single shots (508 x 308, 500 steps) one after another beside 16 served shots
-// on 2108 x 908 (135 ms without them): launches of 256 steps without pauses
-// 7.4 ms a shot, the server 1585 ms; split launches 139 and 138; this 33 and
-// 166.  Beside 24 served shots on 508 x 308 (103 ms): 7.2 and 1278, 36 and 116,
-// 34 and 125.
+// third of the device's time: launches of kServedSteps steps, each followed by
+// kServedPause times its own duration for the server.  Measured on one B200,
+// single shots (508 x 308, 500 steps, 7.1 ms alone) one after another beside
+// 16 served shots on 2108 x 908 (135 ms without them): launches of 256 steps
+// without pauses 7.4 ms a shot, the server 1585 ms; split launches 139 and
+// 138; this 25 and 178.  Beside 24 served shots on 508 x 308 (103 ms): 7.2 and 1278,
+// 36 and 116, 25 and 133.
 using HostClock = std::chrono::steady_clock;
-constexpr int kServedSteps = 32, kServedPause = 3;
+constexpr int kServedSteps = 32, kServedPause = 2;
 constexpr auto kServedPauseMax = std::chrono::milliseconds(100);  // a launch that itself waited long
 
 template <int M>

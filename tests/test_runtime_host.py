@@ -129,8 +129,8 @@ with F.ShotServer() as srv:
     s.advance(40)                                         # the served shot is in flight: launches of 32 steps
     assert get("launches:resident_kernel") == 2
     put("launch_us", 20000)
-    s.advance(70)                                         # three launches, the first two with pauses of three times their time
-    assert get("launches:resident_kernel") == 5 and time.time() - t0 > 2 * 0.06 + 3 * 0.02
+    s.advance(70)                                         # three launches, the first two with pauses of twice their time
+    assert get("launches:resident_kernel") == 5 and time.time() - t0 > 2 * 0.04 + 3 * 0.02
     put("launch_us", 0)
     put("hold", 0)
     srv.wait(t, timeout=60)
