@@ -17,6 +17,7 @@
 #include <cstring>
 #include <map>
 #include <memory>
+#include <set>
 #include <tuple>
 #include <utility>
 #include <mutex>
@@ -790,7 +791,9 @@ constexpr int kStepTuneWindow = 24;  // steps timed per candidate
 // The optional cache file of step-kernel choices (environment variable
 // FOMO_B200_TUNE_CACHE).  Single-shot kernel choices are lines
 // "step nx nz M nbc fs iso choice", read on first use and appended to when a
-// choice is made; the shot server's lines have five numbers (server.cuh).
+// choice is made; the shot server's lines have five numbers (server.cuh).  A
+// line that ends in a word notes what ran without having been timed: it is
+// not read.
 const char* tune_cache_path() {
     const char* p = std::getenv("FOMO_B200_TUNE_CACHE");
     return (p && *p) ? p : nullptr;
@@ -805,31 +808,32 @@ void load_step_choices() {
     if (!path) return;
     FILE* f = std::fopen(path, "r");
     if (!f) return;
-    char line[256];
+    char line[256], word[16];
     StepKey k;
     int c;
     while (std::fgets(line, sizeof(line), f))
-        if (std::sscanf(line, "step %d %d %d %d %d %d %d", &k.nx, &k.nz, &k.M, &k.nbc, &k.fs, &k.iso, &c) == 7)
+        if (std::sscanf(line, "step %d %d %d %d %d %d %d %15s", &k.nx, &k.nz, &k.M, &k.nbc, &k.fs, &k.iso, &c, word) == 7)
             g_step_choice[k] = c != 0;
     std::fclose(f);
 }
 
-void save_step_choice(const StepKey& k, int c) {
+void save_step_choice(const StepKey& k, int c, const char* word = "") {
     const char* path = tune_cache_path();
     if (!path) return;
     if (FILE* f = std::fopen(path, "a")) {
-        std::fprintf(f, "step %d %d %d %d %d %d %d\n", k.nx, k.nz, k.M, k.nbc, k.fs, k.iso, c);
+        std::fprintf(f, "step %d %d %d %d %d %d %d%s\n", k.nx, k.nz, k.M, k.nbc, k.fs, k.iso, c, word);
         std::fclose(f);
     }
 }
 
-// Records, once per process and grid, that a grid does not run the fused step
-// (it runs the resident kernel, which needs no timing).
-void note_step_choice(const StepKey& k) {
-    if (k.M > 4 || !k.fs) return;  // the fused step never applies there: nothing to choose
+// Notes in the cache file, once per process and grid, that a grid which the
+// fused step could run runs the resident kernel.  Nothing was timed, so it is
+// no choice between the other two.
+void note_resident(const StepKey& k) {
+    if (k.M > 4 || !k.fs || !tune_cache_path()) return;
+    static std::set<StepKey> noted;
     std::lock_guard<std::mutex> lk(g_step_choice_mu);
-    load_step_choices();
-    if (g_step_choice.emplace(k, 0).second) save_step_choice(k, 0);
+    if (noted.insert(k).second) save_step_choice(k, 0, " resident");
 }
 
 // Steps on the split launches or the fused step, as `mode` (FOMO_STEP_*) says.
@@ -895,7 +899,7 @@ int run_steps_M(Shot& s, Medium& m, Wavefield& w, int n_steps, Profile* prof) {
     if (mode == FOMO_STEP_AUTO && !prof) {
         const fomo::ResidentPlan res = shot_resident_plan<M>(s, m);
         if (res.ok) {
-            note_step_choice(StepKey{m.nx, m.nz, M, s.nbc, m.fs, s.dtx == s.dtz});
+            note_resident(StepKey{m.nx, m.nz, M, s.nbc, m.fs, s.dtx == s.dtz});
             bool refused = false;
             do {
                 while (g_served.load() > 0 && HostClock::now() < C.resident_after)

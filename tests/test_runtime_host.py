@@ -27,6 +27,7 @@ b = F.backend("b200")
 case = lambda nx=150, nz=90, **kw: layered(nx, nz, seed=4, **dict(dict(nbc=12, fd_order=8, nt=600), **kw))
 SPLIT = "13stress_kernel"
 MARCH = "12march_kernel"
+def steps(): return get("launches:" + SPLIT) + get("launches:" + MARCH)  # of the split launches and the fused step
 """
 
 
@@ -62,19 +63,19 @@ assert get("launches:resident_kernel") == 3 and get("launches:" + SPLIT) == 0
 
 
 @pytest.mark.parametrize("after", [0, 1])
-def test_refused_cooperative_launch_runs_the_split_launches(host_run, after):
+def test_refused_cooperative_launch_runs_other_launches(host_run, after):
     host_run(f"""
 put("refuse_cooperative_after", {after})
 s = OpenShot(case(), b)
 s.advance(600)
 assert s.k.value == 600
 assert get("launches:resident_kernel") == {after}
-assert get("launches:" + SPLIT) == 600 - 256 * {after}
+assert steps() == 600 - 256 * {after}
 s.finish()
 """)
 
 
-def test_no_room_for_the_mailboxes_runs_the_split_launches(host_run):
+def test_no_room_for_the_mailboxes_runs_other_launches(host_run):
     host_run("""
 s = OpenShot(case(), b)
 F.set_step_kernel("split")
@@ -84,7 +85,7 @@ put("fail_alloc_max", 1 << 40); put("fail_alloc_min", 0)
 for _ in range(3):
     s.advance(100)
 assert s.k.value == 301
-assert get("launches:resident_kernel") == 0 and get("launches:" + SPLIT) == 301
+assert get("launches:resident_kernel") == 0 and steps() == 301
 assert get("failed_allocs") == 2                          # one attempt a shot, and its retry after a trim
 s.finish()
 """)
@@ -105,7 +106,7 @@ else:
 assert get("live_bytes") < held
 put("capacity", 1 << 36)
 s.advance(500)                                            # allocated again
-assert s.k.value == 600 and get("launches:" + SPLIT) == 0
+assert s.k.value == 600 and steps() == 0
 s.finish()
 """)
 
@@ -268,3 +269,32 @@ assert get("reserved") - base <= share + (2 << 30)
 assert wait(A, submit(A)) == ""
 A.close()
 """)
+
+
+def test_resident_grid_is_no_timed_choice_in_the_cache_file(host_run, tmp_path):
+    """A grid that ran the resident kernel was not timed: where it does not fit, both other kernels are."""
+    path = tmp_path / "tune.txt"
+    host_run("""
+for _ in range(2):
+    s = OpenShot(case(), b)
+    s.advance(600)
+    s.finish()
+""", FOMO_B200_TUNE_CACHE=str(path))
+    assert path.read_text().split() == ["step", "182", "122", "4", "12", "1", "1", "0", "resident"]
+    host_run("""
+put("sm_count", 2)                                        # a device the grid's three strips do not fit
+s = OpenShot(case(), b)
+s.advance(600)
+assert get("launches:resident_kernel") == 0
+assert get("launches:" + MARCH) >= 24 and get("launches:" + SPLIT) >= 24
+assert steps() == 600
+""", FOMO_B200_TUNE_CACHE=str(path))
+    lines = path.read_text().strip().split("\n")
+    assert len(lines) == 2 and lines[1].split()[:7] == lines[0].split()[:7] and lines[1].split()[7] in ("0", "1")
+    chosen = 600 if lines[1].split()[7] == "1" else 0
+    host_run(f"""
+put("sm_count", 2)                                        # the timed choice is read
+s = OpenShot(case(), b)
+s.advance(600)
+assert get("launches:" + MARCH) == {chosen} and get("launches:" + SPLIT) == 600 - {chosen}
+""", FOMO_B200_TUNE_CACHE=str(path))
