@@ -145,32 +145,35 @@ struct TuneKey {
     }
 };
 std::mutex g_tune_mu;
-std::map<TuneKey, int> g_tune;  // process-wide: (grid, order, batch size) -> index in kStepChoices
+std::map<TuneKey, int> g_tune;  // from the cache file: (grid, order, batch size) -> index in kStepChoices
 
-// Optional file behind the cache (environment variable FOMO_B200_TUNE_CACHE,
-// tune_cache_path): one line "nx nz M shots_log2 K" per decision, read when a
-// server starts and appended to when a choice is made (lines of the
-// single-shot kernel choice, "step ...", are skipped here).  Call with
-// g_tune_mu held.
+// Optional file of choices (environment variable FOMO_B200_TUNE_CACHE,
+// tune_cache_path): lines "nx nz M shots_log2 K", read when a server starts
+// (lines of the single-shot kernel choice, "step ...", are skipped here).  A
+// line that ends in a word notes what ran without having been chosen: it is
+// not read.  Call with g_tune_mu held.
 void load_tune_cache() {
     const char* path = tune_cache_path();
     if (!path) return;
     FILE* f = std::fopen(path, "r");
     if (!f) return;
-    char line[256];
+    char line[256], word[16];
     int nx, nz, M, lg, K;
     while (std::fgets(line, sizeof(line), f))
-        if (std::sscanf(line, "%d %d %d %d %d", &nx, &nz, &M, &lg, &K) == 5)
+        if (std::sscanf(line, "%d %d %d %d %d %15s", &nx, &nz, &M, &lg, &K, word) == 5)
             for (int c = 0; c < 3; ++c)
                 if (kStepChoices[c] == K) g_tune[TuneKey{nx, nz, M, lg}] = c;
     std::fclose(f);
 }
 
-void save_tune_choice(const TuneKey& k, int cand) {
+// Notes in the file, once per process and key, that the default ran.  Call with
+// g_tune_mu held.
+void note_default_steps(const TuneKey& k) {
+    static std::set<TuneKey> noted;
     const char* path = tune_cache_path();
-    if (!path) return;
+    if (!path || !noted.insert(k).second) return;
     if (FILE* f = std::fopen(path, "a")) {
-        std::fprintf(f, "%d %d %d %d %d\n", k.nx, k.nz, k.M, k.shots_log2, kStepChoices[cand]);
+        std::fprintf(f, "%d %d %d %d %d default\n", k.nx, k.nz, k.M, k.shots_log2, kStepChoices[kStepsDefault]);
         std::fclose(f);
     }
 }
@@ -1142,8 +1145,7 @@ class Server {
     }
 
     // Index in kStepChoices of the next chunk (-2: a configured K that is none
-    // of them): the configuration's, the cache file's, or the default, which
-    // is entered in the cache.
+    // of them): the configuration's, the cache file's, or the default.
     int choose(const TuneKey& key) {
         if (cfg_.steps_per_launch > 0) {
             for (int c = 0; c < 3; ++c)
@@ -1151,9 +1153,10 @@ class Server {
             return -2;
         }
         std::lock_guard<std::mutex> lk(g_tune_mu);
-        const auto [it, added] = g_tune.emplace(key, kStepsDefault);
-        if (added) save_tune_choice(key, it->second);
-        return it->second;
+        const auto it = g_tune.find(key);
+        if (it != g_tune.end()) return it->second;
+        note_default_steps(key);
+        return kStepsDefault;
     }
 
     int run_chunk() {

@@ -298,3 +298,20 @@ s = OpenShot(case(), b)
 s.advance(600)
 assert get("launches:" + MARCH) == {chosen} and get("launches:" + SPLIT) == 600 - {chosen}
 """, FOMO_B200_TUNE_CACHE=str(path))
+
+
+def test_steps_per_launch_in_the_cache_file(host_run, tmp_path):
+    """A K in the file is obeyed; the default is noted and not read as a choice."""
+    path = tmp_path / "tune.txt"
+    script = SERVED + """
+with F.ShotServer() as srv:
+    assert wait(srv, submit(srv, F.sim_params(c.dt, 64, c.dx, c.dz, 8))) == ""
+print(get("launches:19batch_stress_kernel"))              # those of one captured graph
+"""
+    assert host_run(script, FOMO_B200_TUNE_CACHE=str(path)).split() == ["8"]
+    assert path.read_text() == "182 122 4 0 8 default\n"
+    path.write_text("182 122 4 0 32 default\n")
+    assert host_run(script, FOMO_B200_TUNE_CACHE=str(path)).split() == ["8"]
+    path.write_text("182 122 4 0 32\n")
+    assert host_run(script, FOMO_B200_TUNE_CACHE=str(path)).split() == ["32"]
+    assert path.read_text() == "182 122 4 0 32\n"
