@@ -41,7 +41,7 @@ struct ResidentArgs {
     ulonglong2* mail;    // mailboxes of the launch's blocks (resident_mail_items each)
     uint32_t tag0;       // step s of the launch (0-based) marks its messages tag0 + s
     int n_steps, k0;     // steps to run; 1-based number of the first
-    float wav[kRMaxSteps + 1];  // source samples of the steps (wav[n_steps] = 0: nothing to add after the last)
+    float wav[kRMaxSteps];  // source samples of the steps
 };
 
 // x halo of a region, as Geo<M>::HX.
