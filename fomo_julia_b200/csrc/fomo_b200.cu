@@ -29,6 +29,7 @@
 #include "../../include/fomo_b200.h"
 #include "step_tiled.cuh"
 #include "march_launch.h"
+#include "mailbox.cuh"
 #include "resident_launch.h"
 #include "step_march.cuh"
 
@@ -137,13 +138,16 @@ struct Shot : Object {
     }
 };
 
+constexpr int kStatusInts = 12;
+
 struct Context {
     std::mutex mu;
     bool inited = false;
     int device = -1;
     cudaStream_t stream = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
-    int* d_status = nullptr;   // device error word of the kernels, then the fused step's work queue (2 ints)
+    int* d_status = nullptr;   // device error word of the kernels, at + 2 the fused step's work queue (2 ints), at + 8 an
+                               // empty mailbox (one message, for the self-test); kStatusInts ints
     cudaMemPool_t pool = nullptr;
     ulonglong2* mail = nullptr;  // mailboxes of the resident kernel, and their number of messages
     size_t mail_items = 0;
@@ -1069,8 +1073,8 @@ int fomo_b200_init(int device) {
     CUDA_TRY(cudaStreamCreateWithFlags(&C.stream, cudaStreamNonBlocking));
     CUDA_TRY(cudaEventCreate(&C.ev0));
     CUDA_TRY(cudaEventCreate(&C.ev1));
-    CUDA_TRY(cudaMalloc(&C.d_status, 4 * sizeof(int)));
-    CUDA_TRY(cudaMemset(C.d_status, 0, 4 * sizeof(int)));
+    CUDA_TRY(cudaMalloc(&C.d_status, kStatusInts * sizeof(int)));
+    CUDA_TRY(cudaMemset(C.d_status, 0, kStatusInts * sizeof(int)));
     cudaMemPoolProps props;
     std::memset(&props, 0, sizeof(props));
     props.allocType = cudaMemAllocationTypePinned;
@@ -1578,7 +1582,13 @@ int fomo_b200_selftest_wait(int32_t polls, int32_t* status) {
     CUDA_TRY(cudaMemsetAsync(ctx().d_status, 0, sizeof(int), st));
     fomo::wait_selftest_kernel<<<1, 32, 0, st>>>(ctx().d_status, polls);
     CUDA_TRY(cudaGetLastError());
-    const int rc = check_status();
+    int rc = check_status();
+    if (rc == FOMO_ETIMEOUT) {  // and a wait of the resident kernel
+        CUDA_TRY(cudaMemsetAsync(ctx().d_status, 0, sizeof(int), st));
+        fomo::mail_selftest_kernel<<<1, 32, 0, st>>>(reinterpret_cast<const ulonglong2*>(ctx().d_status + 8), ctx().d_status, polls);
+        CUDA_TRY(cudaGetLastError());
+        rc = check_status();
+    }
     *status = rc;
     CUDA_TRY(cudaMemsetAsync(ctx().d_status, 0, sizeof(int), st));
     CUDA_TRY(cudaStreamSynchronize(st));

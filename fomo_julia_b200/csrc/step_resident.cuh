@@ -35,22 +35,11 @@
 // and the receivers (source_receiver.jl:18-30, boundary.jl:20-56).
 #pragma once
 
+#include "mailbox.cuh"
 #include "resident_launch.h"
 #include "step_tiled.cuh"
 
 namespace fomo {
-
-// One 16-byte message; each half is written and read as one 64-bit access.
-__device__ __forceinline__ void mail_put(ulonglong2* p, float a, float b, uint32_t tag) {
-    const uint64_t lo = ((uint64_t)tag << 32) | __float_as_uint(a), hi = ((uint64_t)tag << 32) | __float_as_uint(b);
-    asm volatile("st.relaxed.gpu.global.v2.b64 [%0], {%1, %2};" ::"l"(p), "l"(lo), "l"(hi) : "memory");
-}
-__device__ __forceinline__ ulonglong2 mail_get(const ulonglong2* p) {
-    ulonglong2 v;
-    asm volatile("ld.relaxed.gpu.global.v2.b64 {%0, %1}, [%2];" : "=l"(v.x), "=l"(v.y) : "l"(p) : "memory");
-    return v;
-}
-constexpr int kMailPolls = 1 << 22;
 
 // z-derivatives of RT consecutive rows from a (2M + RT - 1)-row window:
 // d[rr] = sum_l a_l (w[rr+M+l-1] - w[rr+M-l]), column pairs.
@@ -772,12 +761,9 @@ __global__ void __launch_bounds__(kRThreads, 1)
                             todo &= ~(1u << q);
                         }
                     }
-                if (todo && ((it & 4095) == 4095)) {  // give up, or follow a block that has
-                    if (it >= kMailPolls || *reinterpret_cast<volatile int*>(A.status) != 0) {
-                        atomicCAS(A.status, 0, kErrResidentTimeout);
-                        s_abort = 1;
-                        todo = 0;
-                    }
+                if (todo && mail_check_due(it) && mail_gives_up(it, kMailPolls, A.status)) {
+                    s_abort = 1;
+                    todo = 0;
                 }
             }
         }

@@ -272,12 +272,14 @@ int fomo_b200_shot_profile(uint64_t shot_handle, int32_t n_steps, FomoKernelTime
 int fomo_b200_set_step_kernel(int32_t mode, int32_t n_segs);
 
 /* Self-test of the kernels' bounded device waits (no reference
- * counterpart).  Every wait of a time-step kernel on its TMA loads polls at
- * most a fixed number of times, then records an error that the call reports
- * as FOMO_ETIMEOUT instead of hanging the GPU.  This runs the same wait on a
- * barrier that nothing completes, for `polls` polls (1..2^20), and stores
- * the resulting status in *status (FOMO_ETIMEOUT when the mechanism works);
- * nothing is left outstanding on the device. */
+ * counterpart).  Every wait of a time-step kernel, on its TMA loads or (the
+ * resident kernel) on its neighbours' messages, polls at most a fixed number
+ * of times, then records an error that the call reports as FOMO_ETIMEOUT
+ * instead of hanging the GPU.  This runs the same waits on a barrier that
+ * nothing completes and on a message that nobody sends, for `polls` polls
+ * each (1..2^20; the second rounded up to 4096), and stores the resulting
+ * status in *status (FOMO_ETIMEOUT when both end so); nothing is left
+ * outstanding on the device. */
 int fomo_b200_selftest_wait(int32_t polls, int32_t* status);
 
 /* Allocation-free shot.  No counterpart in the reference: it exists for

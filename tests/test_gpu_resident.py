@@ -124,3 +124,15 @@ def test_resident_beside_a_busy_server(b200, oracle_lib):
     assert len(out) == 5 and all(np.array_equal(r.gather, ref.gather) for r in out)
     assert all(np.array_equal(r.gather, res[0].gather) for r in res)
     med.release()
+
+
+def test_resident_wait_is_bounded(b200, oracle_lib):
+    """A wait for a message that nobody sends ends with FOMO_ETIMEOUT, whatever the limit, and a shot runs after it."""
+    import ctypes
+    from fomo_julia_b200._lib import call, load
+    st = ctypes.c_int32(0)
+    for polls in (1, 1000, 4097):
+        call("fomo_b200_selftest_wait", polls, ctypes.byref(st))
+        assert st.value == -4
+        assert b"did not hear from its neighbours" in load().fomo_b200_last_error()
+    _check(layered(50, 40, seed=7, nbc=5, fd_order=8, nt=60), b200, oracle_lib)
