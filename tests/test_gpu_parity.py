@@ -251,3 +251,14 @@ def test_invalid_inputs_raise(b200):
     c.rec_z = np.array([0.0], dtype=np.float32)
     with pytest.raises(F._lib.FomoError, match="FOMO_EINVAL.*receiver"):
         gpu_run(c, b200)
+
+
+@pytest.mark.parametrize("c", [c for c in CASES if not fused_supported(c)], ids=lambda c: c.name)
+def test_split_launches_match_oracle_beyond_the_fused_step(c, b200, oracle_lib, step_kernel):
+    # no free surface, orders 10 and 12, wide bands: what larger grids of these kinds run under "auto"
+    # (these small ones run the resident kernel there)
+    step_kernel("split")
+    r, f_gpu = gpu_run(c, b200)
+    g_orc, f_orc = oracle_run(c, oracle_lib)
+    assert_same(r.gather, g_orc, f_gpu, f_orc)
+    assert r.stats["kernel_launches"] >= 4 * c.nt

@@ -111,3 +111,22 @@ def test_saved_gather_after_a_change_of_kernels(b200, step_kernel, tmp_path):
     call("fomo_b200_shot_save_gather", s.handle.value, str(path).encode())
     s.finish()
     assert np.array_equal(F.load_gather(str(path), *ref[0].shape), ref[0])
+
+
+def test_kernels_timed_on_live_steps(b200, step_kernel, tmp_path, monkeypatch):
+    """A grid too large for the resident kernel: its first shot times the fused step and the split launches on 24
+    steps each, records the faster and runs the rest on it."""
+    path = tmp_path / "tune.txt"
+    monkeypatch.setenv("FOMO_B200_TUNE_CACHE", str(path))
+    c = layered(1463, 883, seed=6, nbc=10, fd_order=8, nt=100, n_rec=9)  # 1491 x 911 padded
+    first = whole_shot(c, b200, step_kernel, "auto")
+    line = path.read_text().split()
+    assert line[:7] == ["step", "1491", "911", "4", "10", "1", "1"] and line[7:] in (["0"], ["1"])
+    rest = 1 if line[7] == "1" else 4  # launches per step
+    assert first[2] == 24 + 4 * 24 + rest * 52 + 1  # and the last row's receivers
+    again = whole_shot(c, b200, step_kernel, "auto")
+    assert again[2] == rest * 100 + 1 and path.read_text().split() == line
+    ref = whole_shot(c, b200, step_kernel, "split")
+    assert ref[2] == 401 and np.abs(ref[0]).max() > 0
+    assert_equal(first, ref)
+    assert_equal(again, ref)
