@@ -255,10 +255,14 @@ int fomo_b200_shot_profile(uint64_t shot_handle, int32_t n_steps, FomoKernelTime
  * runs a single shot on the resident kernel where the grid fits; elsewhere
  * it times the other two on 24 live steps each of the first shot of a (grid,
  * order, HABC width) with enough steps left, keeps the faster for the
- * process (and in the FOMO_B200_TUNE_CACHE file when that is set; a grid
- * that runs the resident kernel is entered there as not fused), and runs the
+ * process (and in the FOMO_B200_TUNE_CACHE file when that is set; for a grid
+ * that runs the resident kernel the file gets a line ending in "resident",
+ * which is not read), and runs the
  * split launches where the fused step does not apply or the shot is too
- * short to time.  FOMO_STEP_SPLIT always runs the split
+ * short to time.  A resident grid runs as the others do where its mailboxes
+ * (up to 13 MB) or its cooperative launch cannot be had.  While a shot
+ * server of the process has shots in flight, resident launches take a third
+ * of the device's time.  FOMO_STEP_SPLIT always runs the split
  * launches; FOMO_STEP_FUSED fails a single shot that the fused step does not
  * support with FOMO_EINVAL.  n_segs > 0 fixes the fused step's row segments
  * per column strip (1..64; 0 = chosen from the grid and the SM count).
