@@ -28,7 +28,7 @@
 //   sides   a thread's neighbours in x are in the same half warp, so the side
 //           rules run on registers and shuffles;
 //   bottom  the recurrence along j (boundary.jl:88-132) runs in the plane,
-//           one warp per field, with the step-start values in a scratch;
+//           a column per lane, with the step-start values in a scratch;
 //   top     pointwise on values before the band rule, kept in a scratch.
 // The source is added in the plane right after a step's stresses are final
 // (before they are sent), the values before it are kept beside for the HABC
